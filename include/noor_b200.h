@@ -691,8 +691,7 @@ typedef struct noor_wf_params {
 /* BINARY: both stages on the binary tree; WIDE: both on the four-wide tree
  * where every scene of the launch has one (noor_wide_tree_info);
  * WIDE_SHADOW: extension rays on the binary tree, shadow rays on the
- * four-wide one; AUTO: WIDE_SHADOW when every scene of the launch has a
- * four-wide tree and at least 16384 triangles, else BINARY */
+ * four-wide one; AUTO: WIDE */
 enum {
     NOOR_TRAVERSAL_AUTO = 0,
     NOOR_TRAVERSAL_BINARY = 1,

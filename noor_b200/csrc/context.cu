@@ -261,8 +261,13 @@ void apply_spec(SceneState& st, const noor_spec& s) {
     const bool wide = st.wide_nodes && s.bvh_root_node == st.wide_root;
     D.nodes4 = wide ? st.wide_nodes : nullptr;
     D.map4 = wide ? st.wide_map : nullptr;
+    D.leaf_of = wide ? st.wide_leaf_of : nullptr;
+    D.inst_root = wide ? st.wide_inst_root : nullptr;
+    D.root4 = wide ? st.wide_root_word : 0u;
+    D.reach4 = wide ? st.wide_reach : 0.0f;
     D.stack_cap4 = wide ? st.wide_cap : 0;
     D.closest4 = wide && st.wide_closest ? 1u : 0u;
+    D.mega4 = D.closest4 && st.wide_binary_need <= D.stack_cap ? 1u : 0u;
     D.stack_words = std::max(D.stack_cap, D.stack_cap4);
 }
 
@@ -389,6 +394,18 @@ static int check_scene_inputs(const noor_payload* P, const noor_hosek_sky* H, co
     return NOOR_OK;
 }
 
+// bit i of word i / 32: instance i's world-to-object rows are exactly the identity
+static std::vector<uint32_t> identity_instances(const noor_payload* P) {
+    std::vector<uint32_t> ident(P->num_instances / 32 + 1, 0u);
+    for (size_t i = 0; i < P->num_instances; ++i) {
+        bool id = true;
+        for (int r = 0; r < 3; ++r)
+            for (int c = 0; c < 4; ++c) id = id && P->world_to_object_row[r][4 * i + c] == (r == c ? 1.0f : 0.0f);
+        if (id) ident[i / 32] |= 1u << (i % 32);
+    }
+    return ident;
+}
+
 int upload_scene(Context& C, const noor_payload* P, const noor_hosek_sky* H, const noor_spec* S, SceneState& st,
                  bool checked = false) {
     int rc = checked ? NOOR_OK : check_scene_inputs(P, H, S);
@@ -412,14 +429,25 @@ int upload_scene(Context& C, const noor_payload* P, const noor_hosek_sky* H, con
         // the four-wide tree of the spec's root (shadow rays, and closest hit
         // where it qualifies); a tree it does not suit keeps the binary
         // traversal
+        static_assert(sizeof(DevNode4) == sizeof(WideNodeHost), "device wide node");
+        const std::vector<uint32_t> ident = identity_instances(P);
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(h.data());
         WideTree wt;
-        if (build_wide_tree(reinterpret_cast<const uint32_t*>(h.data()), nn, S->bvh_root_node, kWideMaxStack, wt,
-                            nullptr)) {
-            if ((rc = st.upload((void**)&st.wide_nodes, wt.nodes.data(), wt.nodes.size() * sizeof(DevNode4),
+        WideTreeDev wd;
+        if (build_wide_tree(words, nn, S->bvh_root_node, kWideMaxStack, wt, nullptr) &&
+            pack_wide_tree(words, wt, nt, ident, wd)) {
+            if ((rc = st.upload((void**)&st.wide_nodes, wd.nodes.data(), wd.nodes.size() * sizeof(DevNode4),
                                 "wide nodes")) ||
-                (rc = st.upload((void**)&st.wide_map, wt.map.data(), nn * sizeof(uint32_t), "wide map")))
+                (rc = st.upload((void**)&st.wide_map, wt.map.data(), nn * sizeof(uint32_t), "wide map")) ||
+                (rc = st.upload((void**)&st.wide_leaf_of, wd.leaf_of.data(), wd.leaf_of.size() * sizeof(uint32_t),
+                                "wide leaves")) ||
+                (rc = st.upload((void**)&st.wide_inst_root, wd.inst_root.data(), wd.inst_root.size() * sizeof(uint32_t),
+                                "wide instances")))
                 return rc;
+            st.wide_root_word = wd.root_word;
             st.wide_root = wt.root;
+            st.wide_reach = wd.reach;
+            st.wide_binary_need = wt.binary_need;
             st.wide_cap = wt.stack_need;
             st.wide_closest = wt.closest;
         }
@@ -461,15 +489,7 @@ int upload_scene(Context& C, const noor_payload* P, const noor_hosek_sky* H, con
                 std::memcpy(&x[i].nrm[r], P->normal_row[r] + 4 * i, 16);
             }
         if ((rc = st.upload((void**)&D.xforms, x.data(), ni * sizeof(DevXform), "transforms"))) return rc;
-        // instances whose world-to-object rows are exactly the identity
-        std::vector<uint32_t> ident(ni / 32 + 1, 0u);
-        for (size_t i = 0; i < ni; ++i) {
-            const float4* r = x[i].w2o;
-            const bool id = r[0].x == 1.0f && r[0].y == 0.0f && r[0].z == 0.0f && r[0].w == 0.0f &&
-                            r[1].x == 0.0f && r[1].y == 1.0f && r[1].z == 0.0f && r[1].w == 0.0f &&
-                            r[2].x == 0.0f && r[2].y == 0.0f && r[2].z == 1.0f && r[2].w == 0.0f;
-            if (id) ident[i / 32] |= 1u << (i % 32);
-        }
+        const std::vector<uint32_t> ident = identity_instances(P);
         if ((rc = st.upload((void**)&D.xf_ident, ident.data(), ident.size() * 4, "identity instances"))) return rc;
     }
     {

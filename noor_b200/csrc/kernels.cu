@@ -137,8 +137,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_closest(DevScene S, const
     const noor_ray r = rays[i];
     float tmax = r.tmax;
     HitRec rec{0.0f, 0.0f, 0u, 0u, 0u};
-    const bool h = trace_primary<ISECT, true, WIDE>(S, f3(r.org[0], r.org[1], r.org[2]), f3(r.dir[0], r.dir[1], r.dir[2]),
-                                        tmax, rec, st, status);
+    const HeldRay world{f3(r.org[0], r.org[1], r.org[2]), f3(r.dir[0], r.dir[1], r.dir[2])};
+    const bool h = trace_primary<ISECT, true, WIDE>(S, world, tmax, rec, st, status);
     noor_hit o;
     o.t = tmax;
     o.tri_idx = rec.tri;
@@ -159,10 +159,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_any(DevScene S, const noo
     if (i >= n) return;
     SmemStack st{smem + threadIdx.x, (int)blockDim.x, S.stack_cap};
     const noor_ray r = rays[i];
-    occ[i] = trace_shadow<ISECT, true, WIDE>(S, f3(r.org[0], r.org[1], r.org[2]), f3(r.dir[0], r.dir[1], r.dir[2]),
-                                             r.tmax, st, status)
-                 ? 1u
-                 : 0u;
+    const HeldRay world{f3(r.org[0], r.org[1], r.org[2]), f3(r.dir[0], r.dir[1], r.dir[2])};
+    occ[i] = trace_shadow<ISECT, true, WIDE>(S, world, r.tmax, st, status) ? 1u : 0u;
 }
 
 __global__ void k_camera_rays(DevCamera C, uint32_t frame, noor_ray* rays) {

@@ -21,6 +21,11 @@ struct SceneState {
     // the four-wide any-hit tree (wide_bvh.h) and the root it was built from
     const DevNode4* wide_nodes = nullptr;
     const uint32_t* wide_map = nullptr;
+    const uint32_t* wide_leaf_of = nullptr;
+    const uint32_t* wide_inst_root = nullptr;
+    uint32_t wide_root_word = 0;
+    float wide_reach = 0.0f;
+    int wide_binary_need = 0;       // the stack the binary walk of the same tree can need
     uint32_t wide_root = 0;
     int wide_cap = 0;
     bool wide_closest = false;

@@ -16,11 +16,11 @@ struct __align__(32) DevNode {
     uint4 hi;
 };
 
-// Four-wide any-hit node = 128 B (one line): the four entry boxes as
-// structure of arrays, the entry words and meta (wide_bvh.h)
+// Four-wide node = 128 B (one line): the four entry boxes as structure of
+// arrays, the entry words and meta (WideTreeDev in wide_bvh.h)
 struct __align__(128) DevNode4 {
-    float4 lox, loy, loz;
-    float4 hix, hiy, hiz;
+    float4 lo[3];
+    float4 hi[3];
     uint4 child;
     uint4 meta;
 };
@@ -216,8 +216,13 @@ struct DevScene {
     // traversals can need; stack_words = the largest of the stacks
     const DevNode4* nodes4;
     const uint32_t* map4;
+    const uint32_t* leaf_of;    // binary node of the leaf that starts at a triangle
+    const uint32_t* inst_root;  // the word of a transform's tree (kWInstance words)
+    uint32_t root4;             // the word a walk starts from
+    float reach4;               // the largest coordinate of the tree's boxes
     int stack_cap4;
     uint32_t closest4;      // closest hit may use the four-wide tree
+    uint32_t mega4;         // the megakernel and the adjoint may: closest4, and the binary walk's stack fits stack_cap
     int stack_words;
     // NOOR_ENV_REFERENCE: the reference's distribution tables (row r at
     // r * (rw + 1), the marginal at rh * (rw + 1)) and the environment as a

@@ -71,7 +71,8 @@ NB_D bool enter_instance(TRay& lr, const TRay& wr, const DevScene& S, uint32_t i
 }
 
 // slab test of noor/cuda/bbox.cuh:62-80
-NB_D bool slab_hit_f(const TRay& r, float mnx, float mny, float mnz, float mxx, float mxy, float mxz, float tmax) {
+template <class Ray>
+NB_D bool slab_hit_f(const Ray& r, float mnx, float mny, float mnz, float mxx, float mxy, float mxz, float tmax) {
     const bool nx = r.neg & 1u, ny = r.neg & 2u, nz = r.neg & 4u;
     float tMin = xmul(xsub(nx ? mxx : mnx, r.o.x), r.inv.x);
     float tMax = xmul(xsub(nx ? mnx : mxx, r.o.x), r.inv.x);
@@ -87,14 +88,16 @@ NB_D bool slab_hit_f(const TRay& r, float mnx, float mny, float mnz, float mxx, 
     if (tzMax < tMax) tMax = tzMax;
     return (tMin < tmax) && (tMax > 0.0f);
 }
-NB_D bool slab_hit(const TRay& r, const uint4& lo, const uint4& hi, float tmax) {
+template <class Ray>
+NB_D bool slab_hit(const Ray& r, const uint4& lo, const uint4& hi, float tmax) {
     return slab_hit_f(r, __uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(hi.x),
                       __uint_as_float(hi.y), __uint_as_float(hi.z), tmax);
 }
 
 // Wald projection test (noor/cuda/triangle.cuh:82-141); on success writes
 // t into tmax and the barycentrics (u weights v1, v weights v2).
-NB_D bool wald_test(const TRay& r, const DevWaldTri* tri, float& tmax, float& bu, float& bv,
+template <class Ray>
+NB_D bool wald_test(const Ray& r, const DevWaldTri* tri, float& tmax, float& bu, float& bv,
                     uint32_t& mtype) {
     const uint4 a = __ldg(&tri->ax_nu_nv_nd);
     const uint4 c = __ldg(&tri->cnu_cnv_deg_mat);
@@ -149,7 +152,8 @@ NB_D void wt_setup(WtRay& w, const float3& d) {
 
 NB_D float xorsign(float v, uint32_t signbit) { return __uint_as_float(__float_as_uint(v) ^ signbit); }
 
-NB_D bool wt_test(const TRay& r, const WtRay& w, const DevWtTri* tri, float& tmax, float& bu,
+template <class Ray>
+NB_D bool wt_test(const Ray& r, const WtRay& w, const DevWtTri* tri, float& tmax, float& bu,
                   float& bv, uint32_t& mtype) {
     const float4 p0 = __ldg(&tri->v0);
     const float4 p1 = __ldg(&tri->v1);
@@ -521,97 +525,115 @@ NB_D bool trace_any(const DevScene& S, const float3& o, const float3& d, float t
 }
 
 // A ray below which the four-wide tree's boxes may not stand in for the
-// binary tree's: a direction component that is zero, subnormal or NaN (its
-// slab reciprocal is infinite, and the per-axis intervals stop being
-// monotone in the box), or an origin that is not finite.  Such rays walk the
-// binary tree node by node.
+// binary tree's: a direction component that is zero or so small (or an origin
+// or direction so large) that the box test's products could leave the range
+// its error bound covers, or a component that is not a number.  Such rays
+// walk the binary tree node by node.
 NB_D bool wide_degenerate(const float3& o, const float3& d) {
-    const float m = 1.17549435e-38f;  // FLT_MIN
-    return !(fabsf(d.x) >= m && fabsf(d.y) >= m && fabsf(d.z) >= m && fabsf(o.x) <= 3.40282347e38f &&
-             fabsf(o.y) <= 3.40282347e38f && fabsf(o.z) <= 3.40282347e38f);
+    const float lo = 1e-18f, hi = 1e18f, far = kWideMaxCoord;
+    const float3 a = f3(fabsf(d.x), fabsf(d.y), fabsf(d.z));
+    return !(a.x >= lo && a.y >= lo && a.z >= lo && a.x <= hi && a.y <= hi && a.z <= hi && fabsf(o.x) <= far &&
+             fabsf(o.y) <= far && fabsf(o.z) <= far);
 }
 
-NB_D uint32_t word_of(const uint4& v, uint32_t s) { return s == 0 ? v.x : (s == 1 ? v.y : (s == 2 ? v.z : v.w)); }
-NB_D float comp4(const float4& v, uint32_t s) { return s == 0 ? v.x : (s == 1 ? v.y : (s == 2 ? v.z : v.w)); }
+// The level's ray as the wide nodes' box test takes it: a plane at x (on axis
+// a) is met at x * inv[a] + c, c = -o[a] * inv[a] moved down (cn, near
+// planes) or up (cf, far planes) by pad * |inv[a]|, which bounds what rounding
+// adds: in units of the box coordinates, with u = 2^-24 and |x| <= reach, c
+// and x * inv + c round at most u (2 |o| + reach), the exact slab test
+// (x - o) * inv at most u * 2 (|o| + reach), in all below pad = 5 u (|o| +
+// reach).
+template <int ISECT>
+struct BoxRay {
+    float3 o, inv, cn, cf;
+    uint32_t neg;       // bit a set when d[a] <= 0
+};
+template <>
+struct BoxRay<NOOR_ISECT_REF_WALD> {
+    float3 o, inv, cn, cf;
+    uint32_t neg;
+    float3 d;           // the watertight test keeps its own constants of d
+};
 
-// The slab test of noor/cuda/bbox.cuh:62-80 on a wide node's four entry
-// boxes at once, axis by axis: the same operations and comparisons as
-// slab_hit_f for each box, the near and far bounds of an axis picked by
-// address (the ray's sign) instead of per box.  Bit s set when box s passes.
-NB_D uint32_t slab4(const TRay& r, const DevNode4* nd, float tmax) {
-    const float4* b = &nd->lox;  // lox, loy, loz, hix, hiy, hiz
-    float t0[4], t1[4];
-    uint32_t ok = 0xFu;
-    {
-        const uint32_t n = (r.neg & 1u) ? 3u : 0u;
-        const float4 a = __ldg(b + n), c = __ldg(b + (3u - n));
-#pragma unroll
-        for (uint32_t s = 0; s < 4; ++s) {
-            t0[s] = xmul(xsub(comp4(a, s), r.o.x), r.inv.x);
-            t1[s] = xmul(xsub(comp4(c, s), r.o.x), r.inv.x);
-        }
-    }
-    {
-        const uint32_t n = (r.neg & 2u) ? 3u : 0u;
-        const float4 a = __ldg(b + 1 + n), c = __ldg(b + 1 + (3u - n));
-#pragma unroll
-        for (uint32_t s = 0; s < 4; ++s) {
-            const float u0 = xmul(xsub(comp4(a, s), r.o.y), r.inv.y);
-            const float u1 = xmul(xsub(comp4(c, s), r.o.y), r.inv.y);
-            if (t0[s] > u1 || u0 > t1[s]) ok &= ~(1u << s);
-            if (u0 > t0[s]) t0[s] = u0;
-            if (u1 < t1[s]) t1[s] = u1;
-        }
-    }
-    {
-        const uint32_t n = (r.neg & 4u) ? 3u : 0u;
-        const float4 a = __ldg(b + 2 + n), c = __ldg(b + 2 + (3u - n));
-#pragma unroll
-        for (uint32_t s = 0; s < 4; ++s) {
-            const float u0 = xmul(xsub(comp4(a, s), r.o.z), r.inv.z);
-            const float u1 = xmul(xsub(comp4(c, s), r.o.z), r.inv.z);
-            if (t0[s] > u1 || u0 > t1[s]) ok &= ~(1u << s);
-            if (u0 > t0[s]) t0[s] = u0;
-            if (u1 < t1[s]) t1[s] = u1;
-        }
-    }
-#pragma unroll
-    for (uint32_t s = 0; s < 4; ++s)
-        if (!(t0[s] < tmax && t1[s] > 0.0f)) ok &= ~(1u << s);
-    return ok;
+// two floats in a 64-bit register pair, and the two-wide multiply-add of sm_100
+typedef unsigned long long f32x2;
+NB_D f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+NB_D f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+NB_D float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
+NB_D float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+// three-operand minimum and maximum (one instruction on sm_100)
+NB_D float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+NB_D float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
-// A wide node's visit: its entries that pass the slab test (and its
-// deferred ones) in the binary traversal's order for the ray's octant (the
-// node's order table), the first into `next`, the rest pushed so that they
-// come off the stack in order.  False on a stack overflow.
-NB_D bool wide_visit(const DevNode4* nd, const uint4& meta, const TRay& r, float tmax, const SmemStack& st, int cap,
+// A wide node's visit: its entries whose box the ray may meet within tmax in
+// the binary traversal's order for the ray's octant, the first into `next`,
+// the rest pushed so that they come off the stack in order.  False on a stack
+// overflow.
+template <class Ray>
+NB_D bool wide_visit(const DevNode4* nd, const uint4& meta, const Ray& r, float tmax, const SmemStack& st, int cap,
                      int& top, uint32_t& next, uint32_t* status) {
-    const uint4 cw = __ldg(&nd->child);
-    uint32_t inc = slab4(r, nd, tmax);
+    // near and far planes picked by address (the ray's sign), two boxes at a time
+    const ulonglong2* b = reinterpret_cast<const ulonglong2*>(nd->lo);
+    const uint32_t sx = (r.neg & 1u) ? 3u : 0u, sy = (r.neg & 2u) ? 3u : 0u, sz = (r.neg & 4u) ? 3u : 0u;
+    const ulonglong2 nx = __ldg(b + sx), fx = __ldg(b + (3u - sx));
+    const ulonglong2 ny = __ldg(b + 1 + sy), fy = __ldg(b + 1 + (3u - sy));
+    const ulonglong2 nz = __ldg(b + 2 + sz), fz = __ldg(b + 2 + (3u - sz));
+    const uint4 child = __ldg(&nd->child);
+    uint32_t w[4] = {child.x, child.y, child.z, child.w};
+    const f32x2 ix = pack2(r.inv.x, r.inv.x), iy = pack2(r.inv.y, r.inv.y), iz = pack2(r.inv.z, r.inv.z);
+    const f32x2 cnx = pack2(r.cn.x, r.cn.x), cny = pack2(r.cn.y, r.cn.y), cnz = pack2(r.cn.z, r.cn.z);
+    const f32x2 cfx = pack2(r.cf.x, r.cf.x), cfy = pack2(r.cf.y, r.cf.y), cfz = pack2(r.cf.z, r.cf.z);
 #pragma unroll
-    for (uint32_t s = 0; s < 4; ++s) {
-        const uint32_t w = word_of(cw, s);
-        if (w == kWNone) inc &= ~(1u << s);
-        else if ((w & (kWRef | kWUntested)) == (kWRef | kWUntested)) inc |= 1u << s;
+    for (uint32_t h = 0; h < 2; ++h) {
+        const f32x2 tnx = fma2(h ? nx.y : nx.x, ix, cnx), tfx = fma2(h ? fx.y : fx.x, ix, cfx);
+        const f32x2 tny = fma2(h ? ny.y : ny.x, iy, cny), tfy = fma2(h ? fy.y : fy.x, iy, cfy);
+        const f32x2 tnz = fma2(h ? nz.y : nz.x, iz, cnz), tfz = fma2(h ? fz.y : fz.x, iz, cfz);
+        const float tn0 = max3(lo2(tnx), lo2(tny), lo2(tnz)), tf0 = min3(lo2(tfx), lo2(tfy), lo2(tfz));
+        const float tn1 = max3(hi2(tnx), hi2(tny), hi2(tnz)), tf1 = min3(hi2(tfx), hi2(tfy), hi2(tfz));
+        if (!(tn0 <= fminf(tf0, tmax) && tf0 >= 0.0f)) w[2 * h] = kWNone;
+        if (!(tn1 <= fminf(tf1, tmax) && tf1 >= 0.0f)) w[2 * h + 1] = kWNone;
     }
-    if (!inc) return true;
-    const uint32_t oct = r.neg & 7u;
-    const uint32_t order = ((oct & 4u) ? meta.z : meta.y) >> (8u * (oct & 3u));
+    // into the ray's order, nearest first
+    const uint32_t f = meta.y >> (3u * (r.neg & 7u));
+    const uint32_t a0 = f & 1u ? w[1] : w[0], a1 = f & 1u ? w[0] : w[1];
+    const uint32_t a2 = f & 2u ? w[3] : w[2], a3 = f & 2u ? w[2] : w[3];
+    const uint32_t o[4] = {f & 4u ? a2 : a0, f & 4u ? a3 : a1, f & 4u ? a0 : a2, f & 4u ? a1 : a3};
+    if (top + 3 > cap) {
+        // room for every entry is checked at once; near the end of the stack, for the entries there are
+        int k = 0;
+        for (int j = 0; j < 4; ++j) k += o[j] != kWNone;
+        if (top + k - 1 > cap) {
+            atomicOr(status, NOOR_DEV_STACK_OVERFLOW);
+            return false;
+        }
+    }
     // last in order first: each taken word pushes the one held before it
+    next = o[3];
 #pragma unroll
-    for (int j = 3; j >= 0; --j) {
-        const uint32_t s = (order >> (2 * j)) & 3u;
-        if (!((inc >> s) & 1u)) continue;
+    for (int j = 2; j >= 0; --j) {
+        if (o[j] == kWNone) continue;
         if (next != kWNone) {
-            if (top + 1 > cap) {
-                atomicOr(status, NOOR_DEV_STACK_OVERFLOW);
-                return false;
-            }
             st.base[top * st.stride] = next;
             ++top;
         }
-        next = word_of(cw, s);
+        next = o[j];
     }
     return true;
 }
@@ -620,17 +642,17 @@ NB_D bool wide_visit(const DevNode4* nd, const uint4& meta, const TRay& r, float
 // node, or for a ray below which boxes may not be skipped one binary step
 // (the far child pushed, the near one next, as trace_closest takes them).
 // False on a stack overflow or a missing wide node.
-NB_D bool inner_step(const DevScene& S, uint32_t ni, const uint4& lo, const uint4& hi, const TRay& r, bool deg,
+NB_D bool inner_step(const DevScene& S, uint32_t ni, const uint4& lo, const uint4& hi, uint32_t neg_bits, bool deg,
                      const SmemStack& st, int cap, int& top, uint32_t& next, uint32_t* status) {
     if (deg) {
         if (top + 1 > cap) {
             atomicOr(status, NOOR_DEV_STACK_OVERFLOW);
             return false;
         }
-        const bool neg = (r.neg >> (hi.w & NOOR_AXIS_MASK)) & 1u;
-        st.base[top * st.stride] = kWRef | kWUntested | (neg ? ni + 1 : lo.w);
+        const bool neg = (neg_bits >> (hi.w & NOOR_AXIS_MASK)) & 1u;
+        st.base[top * st.stride] = kWRef | (neg ? ni + 1 : lo.w);
         ++top;
-        next = kWRef | kWUntested | (neg ? lo.w : ni + 1);
+        next = kWRef | (neg ? lo.w : ni + 1);
         return true;
     }
     next = __ldg(&S.map4[ni]);
@@ -641,216 +663,157 @@ NB_D bool inner_step(const DevScene& S, uint32_t ni, const uint4& lo, const uint
     return true;
 }
 
-// Any hit over the four-wide tree (S.nodes4, layout in wide_bvh.h): the same
-// answer as trace_any on the binary tree.  Binary nodes (leaves, mesh
-// leaves, instances, light nodes and deferred entries) are taken as the
-// binary traversal takes them; a ref carries kWUntested when its box has not
-// been tested yet.  The stack holds S.stack_cap4 words, the deepest this
-// tree can need.  The walk is kept in an Any4 so that a kernel can advance
-// many rays a step at a time (any4_step) and start a new ray on a lane as
-// soon as its last one ends.
-struct Any4 {
-    TRay wr, lr;        // the world ray, the ray of the level being walked
-    WtRay wt;           // watertight constants of wt_ray's level
-    float tmax;
-    uint32_t next;      // the word taken next
-    int top;
-    bool wdeg, ldeg;    // wide_degenerate of the world / level ray
-    bool wtw;           // wt holds the world ray's constants
-    bool plain;         // ray_plain of the world ray
+// The exact slab test of the leaf whose triangles start at `start`, made when
+// one of them is hit: the leaf's box must pass with the distance the binary
+// traversal would have tested it with.
+template <class Ray>
+NB_D bool leaf_box_hit(const DevScene& S, uint32_t start, const Ray& r, float tmax) {
+    const DevNode* nd = S.nodes + __ldg(&S.leaf_of[start]);
+    return slab_hit(r, __ldg(&nd->lo), __ldg(&nd->hi), tmax);
+}
+
+// The world ray of a walk, held in registers or read again from memory where
+// it is needed again (an instance whose transform is not the identity, a
+// light)
+struct HeldRay {
+    float3 o, d;
+    NB_D void get(float3& oo, float3& dd) const {
+        oo = o;
+        dd = d;
+    }
+};
+struct StoredRay {
+    const float4 *o, *d;
+    NB_D void get(float3& oo, float3& dd) const {
+        const float4 a = *o, b = *d;
+        oo = f3(a);
+        dd = f3(b);
+    }
 };
 
+// The ray of the level being walked, for the four-wide traversals.  The world
+// ray is not kept beside it: it is set up again when a top-level node follows
+// an instance whose transform is not the identity.
 template <int ISECT>
-NB_D void any4_init(Any4& a, const DevScene& S, const float3& o, const float3& d, float tmax) {
-    tray_setup(a.wr, o, d);
-    a.lr = a.wr;
-    a.wdeg = a.ldeg = wide_degenerate(o, d);
-    if (ISECT == NOOR_ISECT_WATERTIGHT) wt_setup(a.wt, d);
-    a.wtw = true;
-    a.plain = ray_plain(o, d);
-    a.tmax = tmax;
-    a.top = 0;
-    a.next = kWRef | kWUntested | S.root;
-}
+struct LevelRay {
+    BoxRay<ISECT> r;
+    WtRay wt;           // watertight constants
+    bool deg;           // walks the binary tree
+    bool world;         // r is the world ray
 
-enum : int { kAnyRunning = 0, kAnyHit = 1, kAnyMiss = 2, kAnyFailed = 3 };
-
-// One step of the walk: a wide node's visit or one binary node.
-template <int ISECT, bool EXT>
-NB_D int any4_step(Any4& a, const DevScene& S, const SmemStack& st, uint32_t* status) {
-    const int cap = S.stack_cap4;
-    const uint32_t cur = a.next;
-    a.next = kWNone;
-    if (!(cur & kWRef)) {
-        const DevNode4* nd = S.nodes4 + cur;
-        const uint4 meta = __ldg(&nd->meta);
-        if (meta.x & kW4World) {
-            a.lr = a.wr;
-            a.ldeg = a.wdeg;
-            if (ISECT == NOOR_ISECT_WATERTIGHT && !a.wtw) {
-                wt_setup(a.wt, a.wr.d);
-                a.wtw = true;
-            }
-        }
-        if (!wide_visit(nd, meta, a.lr, a.tmax, st, cap, a.top, a.next, status)) return kAnyFailed;
-    } else {
-        const uint32_t ni = cur & kWIndex;
-        const DevNode* nd = S.nodes + ni;
-        const uint4 lo = __ldg(&nd->lo);
-        const uint4 hi = __ldg(&nd->hi);
-        if (hi.w & NOOR_MESH_NODE_MASK) {
-            a.lr = a.wr;
-            a.ldeg = a.wdeg;
-            if (ISECT == NOOR_ISECT_WATERTIGHT && !a.wtw) {
-                wt_setup(a.wt, a.wr.d);
-                a.wtw = true;
-            }
-        }
-        if (!(cur & kWUntested) || slab_hit(a.lr, lo, hi, a.tmax)) {
-            if (!(hi.w & kNodeKindMask)) {
-                if (!inner_step(S, ni, lo, hi, a.lr, a.ldeg, st, cap, a.top, a.next, status)) return kAnyFailed;
-            } else if (hi.w & NOOR_LIGHT_NODE_MASK) {
-                const uint32_t li = hi.w & NOOR_LIGHT_MASK;
-                float tm = a.tmax;
-                if ((int)li < S.num_area_lights &&
-                    shape_hit<EXT, ISECT == NOOR_ISECT_REF_WALD>(S.area_lights[li], a.wr.o, a.wr.d, tm))
-                    return kAnyHit;
-            } else if (hi.w & NOOR_MESH_INSTANCE_MASK) {
-                const bool same = enter_instance(a.lr, a.wr, S, hi.w & NOOR_TRANS_MASK, a.plain);
-                a.ldeg = same ? a.wdeg : wide_degenerate(a.lr.o, a.lr.d);
-                if (ISECT == NOOR_ISECT_WATERTIGHT && !(same && a.wtw)) {
-                    wt_setup(a.wt, a.lr.d);
-                    a.wtw = same;
-                }
-                a.next = kWRef | kWUntested | lo.w;
-            } else if (hi.w & NOOR_MESH_LEAF_MASK) {
-                const uint32_t cnt = hi.w & NOOR_COUNT_MASK;
-                if (a.top + (int)cnt > cap + 1) {
-                    atomicOr(status, NOOR_DEV_STACK_OVERFLOW);
-                    return kAnyFailed;
-                }
-                for (uint32_t i = 1; i < cnt; ++i) {
-                    st.base[a.top * st.stride] = kWRef | kWUntested | (ni + i);
-                    ++a.top;
-                }
-                if (cnt) a.next = kWRef | kWUntested | (ni + cnt);
-            } else {
-                const uint32_t start = lo.w;
-                const uint32_t end = start + (hi.w & NOOR_TRI_COUNT_MASK);
-                for (uint32_t ti = start; ti < end; ++ti) {
-                    float tm = a.tmax, bu, bv;
-                    uint32_t mt;
-                    bool h;
-                    if (ISECT == NOOR_ISECT_WATERTIGHT)
-                        h = wt_test(a.lr, a.wt, S.wtri + ti, tm, bu, bv, mt);
-                    else
-                        h = wald_test(a.lr, S.wald + ti, tm, bu, bv, mt);
-                    if (h && EXT && S.has_alpha && (mt & NOOR_ALPHA) && alpha_cut<ISECT>(S, ti, bu, bv)) h = false;
-                    if (h) return kAnyHit;
-                }
-            }
-        }
+    NB_D bool hit_triangle(const DevScene& S, uint32_t ti, float& t, float& bu, float& bv, uint32_t& mt) const {
+        if constexpr (ISECT == NOOR_ISECT_WATERTIGHT)
+            return wt_test(r, wt, S.wtri + ti, t, bu, bv, mt);
+        else
+            return wald_test(r, S.wald + ti, t, bu, bv, mt);
     }
-    if (a.next == kWNone) {
-        if (a.top == 0) return kAnyMiss;
-        --a.top;
-        a.next = st.base[a.top * st.stride];
+    NB_D void setup(const DevScene& S, const float3& o, const float3& d, bool binary) {
+        TRay t;
+        tray_setup(t, o, d);
+        r.o = o;
+        r.inv = t.inv;
+        r.neg = t.neg;
+        const float e = 3.0e-7f;
+        const float3 pad = f3(e * (fabsf(o.x) + S.reach4) * fabsf(t.inv.x), e * (fabsf(o.y) + S.reach4) * fabsf(t.inv.y),
+                              e * (fabsf(o.z) + S.reach4) * fabsf(t.inv.z));
+        r.cn = f3(fmaf(-o.x, t.inv.x, -pad.x), fmaf(-o.y, t.inv.y, -pad.y), fmaf(-o.z, t.inv.z, -pad.z));
+        r.cf = f3(fmaf(-o.x, t.inv.x, pad.x), fmaf(-o.y, t.inv.y, pad.y), fmaf(-o.z, t.inv.z, pad.z));
+        deg = binary || wide_degenerate(o, d);
+        if constexpr (ISECT == NOOR_ISECT_WATERTIGHT)
+            wt_setup(wt, d);
+        else
+            r.d = d;
     }
-    return kAnyRunning;
-}
+    template <class World>
+    NB_D void to_world(const DevScene& S, const World& w, bool binary) {
+        if (world) return;
+        float3 o, d;
+        w.get(o, d);
+        setup(S, o, d, binary);
+        world = true;
+    }
+    // into instance `ins`: an instance whose world-to-object rows are exactly
+    // the identity (DevScene::xf_ident) leaves a plain ray as it is
+    template <class World>
+    NB_D void to_object(const DevScene& S, const World& w, uint32_t ins, bool binary) {
+        TRay t, x;
+        w.get(t.o, t.d);
+        if (((__ldg(&S.xf_ident[ins >> 5]) >> (ins & 31u)) & 1u) && ray_plain(t.o, t.d)) {
+            to_world(S, w, binary);
+            return;
+        }
+        tray_to_object(x, t, S.xforms + ins);
+        setup(S, x.o, x.d, binary);
+        world = false;
+    }
+};
 
-template <int ISECT, bool EXT = true>
-NB_D bool trace_any4(const DevScene& S, const float3& o, const float3& d, float tmax, const SmemStack& st,
+// Any hit over the four-wide tree (S.nodes4, layout in wide_bvh.h): the same
+// answer as trace_any on the binary tree.  Refs (mesh leaves, instances,
+// light nodes, deferred entries, leaves a word cannot hold) are taken as the
+// binary traversal takes them.  `binary`: walk the binary tree only (a scene
+// without a four-wide tree, or one whose binary stack may not fit `cap`).
+// The stack holds `cap` words.
+template <int ISECT, bool EXT, class World>
+NB_D bool trace_any4(const DevScene& S, const World& world, float tmax, const SmemStack& st, int cap, bool binary,
                      uint32_t* status) {
-    Any4 a;
-    any4_init<ISECT>(a, S, o, d, tmax);
-    for (;;) {
-        const int r = any4_step<ISECT, EXT>(a, S, st, status);
-        if (r != kAnyRunning) return r == kAnyHit;
+    LevelRay<ISECT> L;
+    {
+        float3 o, d;
+        world.get(o, d);
+        L.setup(S, o, d, binary);
     }
-}
-
-// Closest hit over the four-wide tree: the same hit, to the bit, as
-// trace_closest.  Leaves are taken in the binary traversal's order, and
-// every binary node (leaf, mesh leaf, instance, light) is slab-tested when it
-// is taken, against the hit distance of that moment, as the binary traversal
-// tests it; a wide node's tests only skip entries that the binary traversal
-// would find missed later (its hit distance only shrinks, and a box inside a
-// missed box is missed).  The stack holds S.stack_cap4 words.
-template <int ISECT, bool EXT = true>
-NB_D bool trace_closest4(const DevScene& S, const float3& o, const float3& d, float& tmax, HitRec& rec,
-                         const SmemStack& st, uint32_t* status) {
-    TRay wr;
-    tray_setup(wr, o, d);
-    const bool wdeg = wide_degenerate(o, d);
-    TRay lr = wr;
-    bool ldeg = wdeg;
-    WtRay wt;
-    if (ISECT == NOOR_ISECT_WATERTIGHT) wt_setup(wt, lr.d);
-    bool wtw = true;  // wt holds the world ray's constants
-    const bool plain = ray_plain(o, d);
-    float ltmax = tmax;
-    uint32_t ins = 0;
-    bool hit = false;
-    const int cap = S.stack_cap4;
+    L.world = true;
     int top = 0;
-    uint32_t next = kWRef | S.root;
+    uint32_t next = L.deg ? kWRef | S.root : S.root4;
     for (;;) {
         const uint32_t cur = next;
         next = kWNone;
         if (!(cur & kWRef)) {
             const DevNode4* nd = S.nodes4 + cur;
             const uint4 meta = __ldg(&nd->meta);
-            if (meta.x & kW4World) {
-                lr = wr;
-                ltmax = tmax;
-                ldeg = wdeg;
-                if (ISECT == NOOR_ISECT_WATERTIGHT && !wtw) {
-                    wt_setup(wt, wr.d);
-                    wtw = true;
+            if (meta.x & kW4World) L.to_world(S, world, binary);
+            if (!wide_visit(nd, meta, L.r, tmax, st, cap, top, next, status)) return false;
+        } else if ((cur & (kWUntested | kWLeaf)) == kWLeaf) {
+            const uint32_t start = cur & kWLeafStart, end = start + ((cur >> kWLeafShift) & (kWLeafMaxCount - 1u)) + 1u;
+            for (uint32_t ti = start; ti < end; ++ti) {
+                float tm = tmax, bu, bv;
+                uint32_t mt;
+                bool h = L.hit_triangle(S, ti, tm, bu, bv, mt);
+                if (h && EXT && S.has_alpha && (mt & NOOR_ALPHA) && alpha_cut<ISECT>(S, ti, bu, bv)) h = false;
+                if (h) {
+                    if (leaf_box_hit(S, start, L.r, tmax)) return true;
+                    break;
                 }
             }
-            if (!wide_visit(nd, meta, lr, ltmax, st, cap, top, next, status)) return hit;
+        } else if (cur & kWUntested) {
+            L.to_object(S, world, cur & kWIndex, binary);
+            next = __ldg(&S.inst_root[cur & kWIndex]);
         } else {
             const uint32_t ni = cur & kWIndex;
             const DevNode* nd = S.nodes + ni;
             const uint4 lo = __ldg(&nd->lo);
             const uint4 hi = __ldg(&nd->hi);
-            if (hi.w & NOOR_MESH_NODE_MASK) {
-                lr = wr;
-                ltmax = tmax;
-                ldeg = wdeg;
-                if (ISECT == NOOR_ISECT_WATERTIGHT && !wtw) {
-                    wt_setup(wt, wr.d);
-                    wtw = true;
-                }
-            }
-            if (slab_hit(lr, lo, hi, ltmax)) {
+            if (hi.w & NOOR_MESH_NODE_MASK) L.to_world(S, world, binary);
+            if (slab_hit(L.r, lo, hi, tmax)) {
                 if (!(hi.w & kNodeKindMask)) {
-                    if (!inner_step(S, ni, lo, hi, lr, ldeg, st, cap, top, next, status)) return hit;
+                    if (!inner_step(S, ni, lo, hi, L.r.neg, L.deg, st, cap, top, next, status)) return false;
                 } else if (hi.w & NOOR_LIGHT_NODE_MASK) {
                     const uint32_t li = hi.w & NOOR_LIGHT_MASK;
+                    float tm = tmax;
+                    float3 o, d;
+                    world.get(o, d);
                     if ((int)li < S.num_area_lights &&
-                        shape_hit<EXT, ISECT == NOOR_ISECT_REF_WALD>(S.area_lights[li], o, d, tmax)) {
-                        hit = true;
-                        rec.ins = li;
-                        rec.mtype = NOOR_MESHLIGHT | NOOR_EMITTER;
-                    }
+                        shape_hit<EXT, ISECT == NOOR_ISECT_REF_WALD>(S.area_lights[li], o, d, tm))
+                        return true;
                 } else if (hi.w & NOOR_MESH_INSTANCE_MASK) {
-                    ins = hi.w & NOOR_TRANS_MASK;
-                    const bool same = enter_instance(lr, wr, S, ins, plain);
-                    ltmax = tmax;
-                    ldeg = same ? wdeg : wide_degenerate(lr.o, lr.d);
-                    if (ISECT == NOOR_ISECT_WATERTIGHT && !(same && wtw)) {
-                        wt_setup(wt, lr.d);
-                        wtw = same;
-                    }
+                    L.to_object(S, world, hi.w & NOOR_TRANS_MASK, binary);
                     next = kWRef | lo.w;
                 } else if (hi.w & NOOR_MESH_LEAF_MASK) {
                     const uint32_t cnt = hi.w & NOOR_COUNT_MASK;
                     if (top + (int)cnt > cap + 1) {
                         atomicOr(status, NOOR_DEV_STACK_OVERFLOW);
-                        return hit;
+                        return false;
                     }
                     for (uint32_t i = 1; i < cnt; ++i) {
                         st.base[top * st.stride] = kWRef | (ni + i);
@@ -860,37 +823,132 @@ NB_D bool trace_closest4(const DevScene& S, const float3& o, const float3& d, fl
                 } else {
                     const uint32_t start = lo.w;
                     const uint32_t end = start + (hi.w & NOOR_TRI_COUNT_MASK);
-                    bool leaf_hit = false;
                     for (uint32_t ti = start; ti < end; ++ti) {
-                        float bu, bv;
+                        float tm = tmax, bu, bv;
                         uint32_t mt;
-                        bool h;
-                        if (EXT && S.has_alpha) {
-                            float tc = ltmax;
-                            if (ISECT == NOOR_ISECT_WATERTIGHT)
-                                h = wt_test(lr, wt, S.wtri + ti, tc, bu, bv, mt);
-                            else
-                                h = wald_test(lr, S.wald + ti, tc, bu, bv, mt);
-                            if (h && (mt & NOOR_ALPHA) && alpha_cut<ISECT>(S, ti, bu, bv)) h = false;
-                            if (h) ltmax = tc;
-                        } else if (ISECT == NOOR_ISECT_WATERTIGHT) {
-                            h = wt_test(lr, wt, S.wtri + ti, ltmax, bu, bv, mt);
-                        } else {
-                            h = wald_test(lr, S.wald + ti, ltmax, bu, bv, mt);
-                        }
-                        if (h) {
-                            leaf_hit = true;
-                            rec.u = bu;
-                            rec.v = bv;
-                            rec.tri = ti;
-                            rec.mtype = mt;
-                        }
+                        bool h = L.hit_triangle(S, ti, tm, bu, bv, mt);
+                        if (h && EXT && S.has_alpha && (mt & NOOR_ALPHA) && alpha_cut<ISECT>(S, ti, bu, bv)) h = false;
+                        if (h) return true;
                     }
-                    if (leaf_hit) {
-                        hit = true;
-                        tmax = ltmax;
-                        rec.ins = ins;
+                }
+            }
+        }
+        if (next == kWNone) {
+            if (top == 0) return false;
+            --top;
+            next = st.base[top * st.stride];
+        }
+    }
+}
+
+// Closest hit over the four-wide tree: the same hit, to the bit, as
+// trace_closest.  Leaves are taken in the binary traversal's order.  A ref is
+// slab-tested when it is taken and a leaf when a triangle of it is hit, both
+// against the hit distance of the moment they were taken, as the binary
+// traversal tests them; the quantized boxes only skip what the binary
+// traversal would find missed (its hit distance only shrinks, and a box
+// inside a missed box is missed).
+template <int ISECT, bool EXT, class World>
+NB_D bool trace_closest4(const DevScene& S, const World& world, float& tmax, HitRec& rec, const SmemStack& st, int cap,
+                         bool binary, uint32_t* status) {
+    LevelRay<ISECT> L;
+    {
+        float3 o, d;
+        world.get(o, d);
+        L.setup(S, o, d, binary);
+    }
+    L.world = true;
+    // the distance the level's boxes and triangles are tested with: a light
+    // hit shortens tmax, and the level's follows at the next top-level node
+    float ltmax = tmax;
+    uint32_t ins = 0;
+    bool hit = false;
+    int top = 0;
+    uint32_t next = L.deg ? kWRef | S.root : S.root4;
+    for (;;) {
+        const uint32_t cur = next;
+        next = kWNone;
+        if (!(cur & kWRef)) {
+            const DevNode4* nd = S.nodes4 + cur;
+            const uint4 meta = __ldg(&nd->meta);
+            if (meta.x & kW4World) {
+                L.to_world(S, world, binary);
+                ltmax = tmax;
+            }
+            if (!wide_visit(nd, meta, L.r, ltmax, st, cap, top, next, status)) return hit;
+        } else {
+            uint32_t start = 0, end = 0;
+            bool known = false;   // the leaf's box has passed
+            if ((cur & (kWUntested | kWLeaf)) == kWLeaf) {
+                start = cur & kWLeafStart;
+                end = start + ((cur >> kWLeafShift) & (kWLeafMaxCount - 1u)) + 1u;
+            } else if (cur & kWUntested) {
+                ins = cur & kWIndex;
+                L.to_object(S, world, ins, binary);
+                ltmax = tmax;
+                next = __ldg(&S.inst_root[ins]);
+            } else {
+                const uint32_t ni = cur & kWIndex;
+                const DevNode* nd = S.nodes + ni;
+                const uint4 lo = __ldg(&nd->lo);
+                const uint4 hi = __ldg(&nd->hi);
+                if (hi.w & NOOR_MESH_NODE_MASK) {
+                    L.to_world(S, world, binary);
+                    ltmax = tmax;
+                }
+                if (slab_hit(L.r, lo, hi, ltmax)) {
+                    if (!(hi.w & kNodeKindMask)) {
+                        if (!inner_step(S, ni, lo, hi, L.r.neg, L.deg, st, cap, top, next, status)) return hit;
+                    } else if (hi.w & NOOR_LIGHT_NODE_MASK) {
+                        const uint32_t li = hi.w & NOOR_LIGHT_MASK;
+                        float3 o, d;
+                        world.get(o, d);
+                        if ((int)li < S.num_area_lights &&
+                            shape_hit<EXT, ISECT == NOOR_ISECT_REF_WALD>(S.area_lights[li], o, d, tmax)) {
+                            hit = true;
+                            rec.ins = li;
+                            rec.mtype = NOOR_MESHLIGHT | NOOR_EMITTER;
+                        }
+                    } else if (hi.w & NOOR_MESH_INSTANCE_MASK) {
+                        ins = hi.w & NOOR_TRANS_MASK;
+                        L.to_object(S, world, ins, binary);
+                        ltmax = tmax;
+                        next = kWRef | lo.w;
+                    } else if (hi.w & NOOR_MESH_LEAF_MASK) {
+                        const uint32_t cnt = hi.w & NOOR_COUNT_MASK;
+                        if (top + (int)cnt > cap + 1) {
+                            atomicOr(status, NOOR_DEV_STACK_OVERFLOW);
+                            return hit;
+                        }
+                        for (uint32_t i = 1; i < cnt; ++i) {
+                            st.base[top * st.stride] = kWRef | (ni + i);
+                            ++top;
+                        }
+                        if (cnt) next = kWRef | (ni + cnt);
+                    } else {
+                        start = lo.w;
+                        end = start + (hi.w & NOOR_TRI_COUNT_MASK);
+                        known = true;
                     }
+                }
+            }
+            const float tleaf = ltmax;
+            for (uint32_t ti = start; ti < end; ++ti) {
+                float tc = ltmax, bu, bv;
+                uint32_t mt;
+                bool h = L.hit_triangle(S, ti, tc, bu, bv, mt);
+                // the hit distance is kept only past the alpha cut
+                if (EXT && S.has_alpha && h && (mt & NOOR_ALPHA) && alpha_cut<ISECT>(S, ti, bu, bv)) h = false;
+                if (h) {
+                    if (!known && !leaf_box_hit(S, start, L.r, tleaf)) break;
+                    known = true;
+                    hit = true;
+                    tmax = ltmax = tc;
+                    rec.u = bu;
+                    rec.v = bv;
+                    rec.tri = ti;
+                    rec.mtype = mt;
+                    rec.ins = ins;
                 }
             }
         }
@@ -905,19 +963,22 @@ NB_D bool trace_closest4(const DevScene& S, const float3& o, const float3& d, fl
 
 // Closest hit on the four-wide tree (WIDE: the kernel is launched only for
 // scenes with S.closest4 set) or on the binary one
-template <int ISECT, bool EXT, bool WIDE>
-NB_D bool trace_primary(const DevScene& S, const float3& o, const float3& d, float& tmax, HitRec& rec,
-                        const SmemStack& st, uint32_t* status) {
-    if (WIDE) return trace_closest4<ISECT, EXT>(S, o, d, tmax, rec, st, status);
+template <int ISECT, bool EXT, bool WIDE, class World>
+NB_D bool trace_primary(const DevScene& S, const World& world, float& tmax, HitRec& rec, const SmemStack& st,
+                        uint32_t* status) {
+    if (WIDE) return trace_closest4<ISECT, EXT>(S, world, tmax, rec, st, S.stack_cap4, false, status);
+    float3 o, d;
+    world.get(o, d);
     return trace_closest<ISECT, EXT>(S, o, d, tmax, rec, st, status);
 }
 
 // Any hit on the four-wide tree (WIDE: launched only for scenes with
 // S.nodes4 set) or on the binary one
-template <int ISECT, bool EXT, bool WIDE>
-NB_D bool trace_shadow(const DevScene& S, const float3& o, const float3& d, float tmax, const SmemStack& st,
-                       uint32_t* status) {
-    if (WIDE) return trace_any4<ISECT, EXT>(S, o, d, tmax, st, status);
+template <int ISECT, bool EXT, bool WIDE, class World>
+NB_D bool trace_shadow(const DevScene& S, const World& world, float tmax, const SmemStack& st, uint32_t* status) {
+    if (WIDE) return trace_any4<ISECT, EXT>(S, world, tmax, st, S.stack_cap4, false, status);
+    float3 o, d;
+    world.get(o, d);
     return trace_any<ISECT, EXT>(S, o, d, tmax, st, status);
 }
 

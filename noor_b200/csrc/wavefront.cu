@@ -147,11 +147,13 @@ struct WfDev {
 #ifndef NB_TRAV_MIN_BLOCKS
 #define NB_TRAV_MIN_BLOCKS 8
 #endif
-// the same for the kernels on the four-wide tree: 8 blocks, 64 registers
-// (their wide visits hold four boxes' slab intervals; on the sky-lit
-// 2.6M-triangle scene 82.7 ms per step against 85.3 at 9 blocks and 84.8 at 7)
+// the same for the kernels on the four-wide tree: 7 blocks, 72 registers (28
+// warps per SM).  At 64 registers extend spills inside the walk: 59.0 ms of
+// extend per 64-sample 1920x1080 frame of 2.6M triangles against 38.7 at 72
+// and 38.6 at 80 (13.1 on a batch of twelve frames at 80, 12.4 at 72); the
+// binary tree's extend took 54.0.
 #ifndef NB_TRAV_MIN_BLOCKS_WIDE
-#define NB_TRAV_MIN_BLOCKS_WIDE 8
+#define NB_TRAV_MIN_BLOCKS_WIDE 7
 #endif
 // minimum resident 256-thread blocks per SM of the shading stage: 3 caps
 // its registers at 85 (24 warps per SM instead of 16 at its natural 128)
@@ -417,16 +419,15 @@ __global__ void __launch_bounds__(kScanThreads) wf_bucket_scan(uint32_t* cnt, ui
 }
 
 template <int ISECT, bool EXT, bool WIDE>
-NB_D void extend_one(const WfDev& W, const DevScene& S, uint32_t slot, const float4& ow,
-                     const SmemStack& stk) {
-    const float4 dw = W.d[slot], bw = W.beta[slot];
-    const float3 o = f3(ow.x, ow.y, ow.z), d = f3(dw.x, dw.y, dw.z);
+NB_D void extend_one(const WfDev& W, const DevScene& S, uint32_t slot, const SmemStack& stk) {
+    float tmax = kInf;
+    HitRec rec{0.0f, 0.0f, 0u, 0u, 0u};
+    const StoredRay ray{W.o + slot, W.d + slot};
+    const bool hit = trace_primary<ISECT, EXT, WIDE>(S, ray, tmax, rec, stk, W.status);
+    const float4 bw = W.beta[slot];
     const uint32_t bb = fbits(bw.w);
     const uint32_t bounce = bb & 0xFFFFu;
     const bool spec = (bb >> 16) & 1u;
-    float tmax = kInf;
-    HitRec rec{0.0f, 0.0f, 0u, 0u, 0u};
-    const bool hit = trace_primary<ISECT, EXT, WIDE>(S, o, d, tmax, rec, stk, W.status);
     const float3 beta = f3(bw.x, bw.y, bw.z);
     if (!hit) {
         // the sky term is added by regen (converged lanes), after the
@@ -438,7 +439,7 @@ NB_D void extend_one(const WfDev& W, const DevScene& S, uint32_t slot, const flo
         if (bounce == 0 || spec) {
             float3 c;
             if (rec.mtype & NOOR_MESHLIGHT) {
-                c = beta * area_le<EXT>(S.area_lights[rec.ins], d);
+                c = beta * area_le<EXT>(S.area_lights[rec.ins], f3(W.d[slot]));
             } else {
                 const uint32_t mi = ISECT == NOOR_ISECT_WATERTIGHT ? __ldg(&S.wtri[rec.tri].attr).w
                                                                    : __ldg(&S.wald[rec.tri].attr).w;
@@ -489,15 +490,14 @@ NB_D const DevScene& slot_scene(const WfDev& W, const DevScene& S1, uint32_t fra
 // false: no scene of the launch has sphere or disk lights
 template <int ISECT, bool MULTI, bool EXT, bool WIDE>
 NB_D void extend_slot(const WfDev& W, const DevScene& S1, uint32_t slot, const SmemStack& stk) {
-    const float4 ow = W.o[slot];
-    const DevScene& S = slot_scene<ISECT, MULTI>(W, S1, fbits(ow.w));
+    const DevScene& S = slot_scene<ISECT, MULTI>(W, S1, MULTI ? fbits(W.o[slot].w) : 0u);
     if (ISECT == kIsectMixed) {
         if (S.isect == NOOR_ISECT_WATERTIGHT)
-            extend_one<NOOR_ISECT_WATERTIGHT, EXT, WIDE>(W, S, slot, ow, stk);
+            extend_one<NOOR_ISECT_WATERTIGHT, EXT, WIDE>(W, S, slot, stk);
         else
-            extend_one<NOOR_ISECT_REF_WALD, EXT, WIDE>(W, S, slot, ow, stk);
+            extend_one<NOOR_ISECT_REF_WALD, EXT, WIDE>(W, S, slot, stk);
     } else {
-        extend_one<ISECT == kIsectMixed ? 0 : ISECT, EXT, WIDE>(W, S, slot, ow, stk);
+        extend_one<ISECT == kIsectMixed ? 0 : ISECT, EXT, WIDE>(W, S, slot, stk);
     }
 }
 
@@ -729,17 +729,17 @@ __global__ void __launch_bounds__(NB_TRAV_THREADS, WIDE ? NB_TRAV_MIN_BLOCKS_WID
         const uint32_t q = W.level >= 3 ? W.sh_perm[i] : i;
         const uint32_t e = W.qshadow[q];
         const uint32_t slot = e >> 1;
-        const float4 so = W.sh_o[q], sd = W.sh_d[q];
+        const float tmax = W.sh_o[q].w;
+        const StoredRay ray{W.sh_o + q, W.sh_d + q};
         const DevScene& S = slot_scene<ISECT, MULTI>(W, S1, MULTI ? fbits(W.o[slot].w) : 0u);
-        const float3 o = f3(so.x, so.y, so.z), d = f3(sd.x, sd.y, sd.z);
         bool occ;
         if (ISECT == kIsectMixed) {
             if (S.isect == NOOR_ISECT_WATERTIGHT)
-                occ = trace_shadow<NOOR_ISECT_WATERTIGHT, EXT, WIDE>(S, o, d, so.w, stk, W.status);
+                occ = trace_shadow<NOOR_ISECT_WATERTIGHT, EXT, WIDE>(S, ray, tmax, stk, W.status);
             else
-                occ = trace_shadow<NOOR_ISECT_REF_WALD, EXT, WIDE>(S, o, d, so.w, stk, W.status);
+                occ = trace_shadow<NOOR_ISECT_REF_WALD, EXT, WIDE>(S, ray, tmax, stk, W.status);
         } else {
-            occ = trace_shadow<ISECT == kIsectMixed ? 0 : ISECT, EXT, WIDE>(S, o, d, so.w, stk, W.status);
+            occ = trace_shadow<ISECT == kIsectMixed ? 0 : ISECT, EXT, WIDE>(S, ray, tmax, stk, W.status);
         }
         if (occ) W.pend[e].w = 0.0f;
     }
@@ -871,13 +871,6 @@ struct WfLaunch {
     bool multi;             // the frames use more than one scene
     bool shade_wide_regs;   // single-scene shade built for 128 registers
 };
-
-// NOOR_TRAVERSAL_AUTO takes the four-wide tree for the shadow rays of scenes
-// of at least this many triangles (on the 36-triangle room the binary tree's
-// single-box visits are cheaper; on the 2.6M-triangle sky scene shadow rays
-// take 11.3 ms per step on the wide tree against 11.7, extension rays 50.2
-// against 48.6, so the extension stage keeps the binary tree)
-constexpr uint32_t kWideAutoTris = 16384;
 
 // shading launches per iteration: one per queue some scene can fill
 static uint32_t shade_launches(const WfDev& W, const WfLaunch& L) {
@@ -1048,18 +1041,19 @@ int wavefront_render(Context& C, const noor_wf_frame* frames, uint32_t n_frames,
     L.grid_queue = (uint32_t)std::max(1, C.sm_count) * 16;
     const uint32_t scene0 = frames[0].scene_id;
     bool multi = false, mixed = false;
-    // the four-wide trees where every scene of the launch has them (and,
-    // for NOOR_TRAVERSAL_AUTO, is large enough for them to pay)
+    // the four-wide trees where every scene of the launch has them.
+    // NOOR_TRAVERSAL_AUTO takes them for both stages and every size: extend
+    // and shadow take 0.68 + 0.22 ms on the 36-triangle room (binary 0.77 +
+    // 0.28), 38.7 + 11.6 ms on 2.6M triangles (54.0 + 18.5)
     if (P.traversal > NOOR_TRAVERSAL_WIDE_SHADOW)
         return set_error(NOOR_ERR_INVALID, "wavefront: bad traversal selector");
-    bool wide_c = P.traversal == NOOR_TRAVERSAL_WIDE, wide_a = P.traversal != NOOR_TRAVERSAL_BINARY;
+    bool wide_c = P.traversal == NOOR_TRAVERSAL_WIDE || P.traversal == NOOR_TRAVERSAL_AUTO, wide_a = P.traversal != NOOR_TRAVERSAL_BINARY;
     L.ext = L.ext_lights = L.env_ref = L.tex = L.diff = false;
     L.kinds = 0;
     for (uint32_t i = 0; i < n_frames; ++i) {
         const DevScene& fs = C.scenes[frames[i].scene_id]->dev;
-        const bool big = P.traversal != NOOR_TRAVERSAL_AUTO || fs.num_tris >= kWideAutoTris;
-        wide_c &= fs.closest4 != 0u && big;
-        wide_a &= fs.nodes4 != nullptr && big;
+        wide_c &= fs.closest4 != 0u;
+        wide_a &= fs.nodes4 != nullptr;
         L.kinds |= fs.shade_kinds;
         multi |= frames[i].scene_id != scene0;
         mixed |= fs.isect != C.scenes[scene0]->dev.isect;

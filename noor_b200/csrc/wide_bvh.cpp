@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <thread>
 
 #include "noor_b200.h"
 
@@ -124,6 +125,7 @@ bool build_wide_tree(const uint32_t* nodes8, size_t nn, uint32_t root, int max_s
         if (out.map[n] == kWNone) {
             out.map[n] = (uint32_t)out.nodes.size();
             out.nodes.emplace_back();
+            out.node.push_back(n);
             work.push_back(n);
         }
         return out.map[n];
@@ -244,11 +246,144 @@ bool build_wide_tree(const uint32_t* nodes8, size_t nn, uint32_t root, int max_s
     }
     out.stack_need = need[root];
     out.root = root;
+    // the binary traversal's stack: one push per inner node, n - 1 per mesh
+    // leaf of n members
+    for (uint32_t n : post) {
+        int v = 0;
+        for (uint32_t i = 0; i < T.num_succ(n); ++i) v = std::max(v, need[T.succ(n, i)]);
+        if (T.kind(n) == kInner) v += 1;
+        if (T.kind(n) == kMeshLeaf && T.count(n)) v += (int)T.count(n) - 1;
+        need[n] = v;
+    }
+    out.binary_need = need[root];
     if (out.stack_need > max_stack) return fail("the four-wide traversal needs a deeper stack than allowed");
     // closest hit re-tests every binary node when it is taken and relies on
     // each entry box being tested against the ray of its parent's visit: no
     // deferred entries
     out.closest = !deferred;
+    return true;
+}
+
+namespace {
+
+// f(first, last) over [0, n) on the host threads
+template <class F>
+void parallel_ranges(size_t n, F f) {
+    const size_t threads = std::min<size_t>(std::max(1u, std::thread::hardware_concurrency()), 16);
+    if (n < (1u << 14) || threads == 1) return f((size_t)0, n);
+    std::vector<std::thread> pool;
+    for (size_t k = 0; k < threads; ++k) pool.emplace_back(f, n * k / threads, n * (k + 1) / threads);
+    for (auto& t : pool) t.join();
+}
+
+}  // namespace
+
+bool pack_wide_tree(const uint32_t* nodes8, WideTree& tree, size_t num_tris, const std::vector<uint32_t>& ident,
+                    WideTreeDev& out) {
+    out = WideTreeDev{};
+    const Tree T{nodes8, tree.map.size()};
+    const size_t n = tree.nodes.size(), ni = 32 * ident.size();
+    out.leaf_of.assign(std::max<size_t>(num_tris, 1), kWNone);
+    out.inst_root.assign(std::max<size_t>(ni, 1), kWNone);
+    auto leaf_fits = [&](uint32_t x) {
+        const uint32_t cnt = T.w1(x) & NOOR_TRI_COUNT_MASK;
+        return T.kind(x) == kTriLeaf && cnt >= 1 && cnt <= kWLeafMaxCount && T.w0(x) <= kWLeafStart &&
+               T.w0(x) < num_tris;
+    };
+    auto claim_leaf = [&](uint32_t x) {
+        if (leaf_fits(x) && out.leaf_of[T.w0(x)] == kWNone) out.leaf_of[T.w0(x)] = x;
+    };
+    // the instance node an entry leads to: itself, or the only member of a
+    // mesh leaf whose box holds it; kWNone where there is none
+    auto instance_of = [&](uint32_t x) {
+        if (T.kind(x) == kMeshLeaf && T.count(x) == 1 && T.contains(x, x + 1)) x = x + 1;
+        return T.kind(x) == kInstance ? x : kWNone;
+    };
+    auto transform = [&](uint32_t x) { return T.w1(x) & NOOR_TRANS_MASK; };
+    // the transform is the identity, and the box holds the tree's: the boxes
+    // of the tree are tested against the same ray as the instance's, and one
+    // that passes is inside it
+    auto same_space = [&](uint32_t x) {
+        const uint32_t t = transform(x);
+        return t < ni && t <= kWIndex && ((ident[t / 32] >> (t % 32)) & 1u) && T.contains(x, T.w0(x));
+    };
+    // an inner node whose children stick out of its box is tested exactly
+    auto inner_word = [&](uint32_t x) {
+        const uint32_t w = tree.map[x];
+        return w != kWNone && T.contains(x, x + 1) && T.contains(x, T.w0(x)) ? w : kWRef | x;
+    };
+    auto tree_word = [&](uint32_t x) -> uint32_t {
+        if (T.kind(x) == kInner) return inner_word(x);
+        if (leaf_fits(x) && out.leaf_of[T.w0(x)] == x)
+            return kWRef | kWLeaf | ((T.w1(x) & NOOR_TRI_COUNT_MASK) - 1u) << kWLeafShift | T.w0(x);
+        const uint32_t i = instance_of(x);
+        if (i != kWNone && same_space(i) && out.inst_root[transform(i)] != kWNone) return kWInstance | transform(i);
+        return kWRef | x;
+    };
+    float reach = 0.0f;
+    std::vector<uint32_t> inst;
+    auto see_entry = [&](uint32_t x) {
+        claim_leaf(x);
+        const uint32_t i = instance_of(x);
+        if (i == kWNone || !same_space(i)) return;
+        claim_leaf(T.w0(i));
+        inst.push_back(i);
+    };
+    see_entry(tree.root);
+    for (const WideNodeHost& h : tree.nodes)
+        for (int s = 0; s < 4; ++s) {
+            if (h.child[s] == kWNone) continue;
+            for (int a = 0; a < 3; ++a) reach = std::max(reach, std::max(std::fabs(h.lo[a][s]), std::fabs(h.hi[a][s])));
+            if ((h.child[s] & (kWRef | kWUntested)) == kWRef) see_entry(h.child[s] & kWIndex);
+        }
+    if (!(reach <= kWideMaxCoord)) return false;
+    out.reach = reach;
+    // one tree per transform
+    std::vector<uint32_t> root_of(out.inst_root.size(), kWNone);
+    for (uint32_t i : inst) {
+        uint32_t& r = root_of[transform(i)];
+        r = r == kWNone || r == T.w0(i) ? T.w0(i) : kWRef;
+    }
+    for (size_t t = 0; t < root_of.size(); ++t) {
+        if (root_of[t] == kWNone || root_of[t] == kWRef) continue;
+        // trees of instances inside instances are taken as refs
+        const uint32_t r = root_of[t];
+        out.inst_root[t] = T.kind(r) == kInner ? inner_word(r) : (T.kind(r) == kTriLeaf ? tree_word(r) : kWRef | r);
+    }
+    out.root_word = tree_word(tree.root);
+    out.nodes.swap(tree.nodes);
+    parallel_ranges(n, [&](size_t b, size_t e) {
+        for (size_t i = b; i < e; ++i) {
+            WideNodeHost& h = out.nodes[i];
+            for (int s = 0; s < 4; ++s) {
+                const uint32_t w = h.child[s];
+                const bool none = w == kWNone, deferred = !none && (w & (kWRef | kWUntested)) == (kWRef | kWUntested);
+                for (int a = 0; a < 3; ++a) {
+                    // a box of the tree's that is inside out (the slab test can still pass
+                    // it) gets the box around it
+                    const float lo = std::min(h.lo[a][s], h.hi[a][s]), hi = std::max(h.lo[a][s], h.hi[a][s]);
+                    h.lo[a][s] = none ? 3.4e38f : (deferred ? -3.4e38f : lo);
+                    h.hi[a][s] = none ? -3.4e38f : (deferred ? 3.4e38f : hi);
+                }
+                if (none) continue;
+                if (!(w & kWRef))
+                    h.child[s] = inner_word(tree.node[w]);
+                else
+                    h.child[s] = deferred ? kWRef | (w & kWIndex) : tree_word(w & kWIndex);
+            }
+            const uint32_t f = h.meta[0];
+            uint32_t flips = 0;
+            for (uint32_t o = 0; o < 8; ++o) {
+                uint32_t k = (o >> ((f >> 4) & 3u)) & 1u ? 4u : 0u;
+                if ((f & kW4ExpandL) && ((o >> ((f >> 6) & 3u)) & 1u)) k |= 1u;
+                if ((f & kW4ExpandR) && ((o >> ((f >> 8) & 3u)) & 1u)) k |= 2u;
+                flips |= k << (3 * o);
+            }
+            h.meta[0] = f & kW4World;
+            h.meta[1] = flips;
+            h.meta[2] = h.meta[3] = 0;
+        }
+    });
     return true;
 }
 

@@ -371,9 +371,11 @@ int noor_device_count(int* count);
  * distant_light.  Returns how many were written (<= n). */
 int noor_abi_sizes(uint32_t* out, int n);
 
-/* Render frames *frame_count .. *frame_count+n_frames-1 in one launch of the
- * plain megakernel (one path per (pixel, frame)) and fold them into the film
- * in frame order; *frame_count += n_frames. */
+/* Render frames *frame_count .. *frame_count+n_frames-1 (one path per (pixel,
+ * frame)) and fold them into the film in frame order; *frame_count +=
+ * n_frames.  Staged over the paths of up to 2^22 pixels x frames at a time;
+ * frames beyond that, or without the memory for it, take the megakernel (the
+ * same film). */
 int noor_render_frames(unsigned int* frame_count, unsigned int n_frames);
 /* Film readback: rgba = mean of the folded samples (w = 1). */
 int noor_get_framebuffer(float* host_rgba, size_t n_pixels);

@@ -21,7 +21,8 @@ CSRC = PKG / "csrc"
 OUT = PKG / "libnoor_b200.so"
 OBJ = ROOT / "_build" / "noor_b200"
 
-CU_SOURCES = ["kernels.cu", "envmap.cu", "context.cu", "wavefront.cu", "adjoint.cu", "noalloc.cu", "tonemap.cu",
+CU_SOURCES = ["megakernel_wt.cu", "megakernel_wald.cu", "path_stages_wt.cu", "path_stages_wald.cu",
+              "path_stages.cu", "kernels.cu", "envmap.cu", "context.cu", "wavefront.cu", "adjoint.cu", "noalloc.cu", "tonemap.cu",
               "bvh_gpu.cu"]
 # the GPU BVH builder rounds its split search as the host builder does
 CU_EXTRA = {"bvh_gpu.cu": ["-fmad=false"]}

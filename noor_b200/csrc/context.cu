@@ -107,7 +107,7 @@ Context::~Context() {
     if (stream) cudaStreamSynchronize(stream);
     scenes.clear();
     for (void* p : {(void*)film_sum, (void*)film_comp, (void*)film_out, (void*)part_sum, (void*)part_comp,
-                    (void*)lookat, (void*)status, (void*)counters, (void*)scratch, adj_buf})
+                    (void*)lookat, (void*)status, (void*)counters, (void*)scratch, adj_buf, stage_buf})
         if (p) cudaFree(p);
     for (auto& e : events)
         if (e) cudaEventDestroy(e);
@@ -668,7 +668,8 @@ int need_ctx(Context*& C) {
     return NOOR_OK;
 }
 
-// render frames [frame0, frame0 + n) with the megakernel
+// render frames [frame0, frame0 + n): staged (path_stages.cuh), or with the
+// megakernel where the staged renderer has no room for a frame's paths
 int render_frames(Context& C, uint32_t frame0, uint32_t n) {
     if (n == 0) return NOOR_OK;
     if (frame0 == 0) return set_error(NOOR_ERR_INVALID, "frame numbers start at 1");
@@ -696,9 +697,13 @@ int render_frames(Context& C, uint32_t frame0, uint32_t n) {
     a.lookat = C.lookat;
     a.status = C.status;
     a.counters = C.counters;
-    cudaError_t e = launch_megakernel(st.dev, C.cam, a, C.stream);
-    if (e != cudaSuccess) return cuda_fail(e, "megakernel");
-    C.launches += chunks > 1 ? 2 : 1;
+    bool staged = false;
+    if ((rc = render_staged(C, st.dev, a, &staged))) return rc;
+    if (!staged) {
+        cudaError_t e = launch_megakernel(st.dev, C.cam, a, C.stream);
+        if (e != cudaSuccess) return cuda_fail(e, "megakernel");
+        C.launches += chunks > 1 ? 2 : 1;
+    }
     C.film_count = (frame0 == 1) ? n : C.film_count + n;
     C.last_frame = frame0 + n - 1;
     return NOOR_OK;

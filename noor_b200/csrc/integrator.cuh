@@ -463,11 +463,19 @@ NB_D RayDiff spawn_diff(const Isect& I, const HitDiff& h, const RayDiff& in, con
 // Builds the hit record of CudaIntersection (intersection.cuh:319-377).
 // With `to`, also the texture coordinates and derivatives of TangentOut
 // (I.uv: the barycentrics on an emitter, whose record stops before them).
-template <int ISECT, bool EXT = true>
+// STAGE: for the staged renderer, whose shading has to round as the
+// megakernel's: there the length of d is z z + (y y + x x), each sum fused.
+NB_D float stage_length2(const float3& d) {
+    return __fmaf_rn(d.z, d.z, __fmaf_rn(d.y, d.y, __fmul_rn(d.x, d.x)));
+}
+template <int ISECT, bool EXT = true, bool STAGE = false>
 NB_D void make_isect(const DevScene& S, const float3& o, const float3& d, float t, const HitRec& rec, Isect& I,
                      TangentOut* to = nullptr) {
     I.p = o + t * d;
-    I.wo = normalize_fast(-1.0f * d);
+    if (STAGE)
+        I.wo = (-1.0f * d) * rsqrtf(stage_length2(d));
+    else
+        I.wo = normalize_fast(-1.0f * d);
     I.mtype = rec.mtype;
     I.lobe = lobe_of<EXT>(rec.mtype);
     if (to) I.uv = f2(rec.u, rec.v);

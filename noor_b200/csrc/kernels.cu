@@ -1,103 +1,16 @@
-// Render and parity kernels: the plain megakernel (one path per
-// (pixel, frame), noor/cuda/path_tracer.cu:77-100), the film fold, ray-batch
-// traversal and the device-routine evaluators used by the parity tests.
+// Render and parity kernels: the film fold, ray-batch traversal and the
+// device-routine evaluators used by the parity tests (the megakernel is in
+// megakernel.cuh).
 #include "kernels.h"
 #include "integrator.cuh"
 
 namespace nb {
-
-// warp-aggregated add of per-lane counts into a 64-bit device counter
-NB_D void warp_count(unsigned long long* ctr, uint32_t v) {
-    const uint32_t mask = __activemask();
-    const uint32_t s = __reduce_add_sync(mask, v);
-    const int leader = __ffs(mask) - 1;
-    if ((int)(threadIdx.x & 31) == leader && s) atomicAdd(ctr, (unsigned long long)s);
-}
 
 NB_D void kahan_add(float3& sum, float3& c, const float3& x) {
     const float3 y = x - c;
     const float3 t = sum + y;
     c = (t - sum) - y;
     sum = t;
-}
-
-// minimum resident blocks per SM the megakernel is compiled for: 7 caps its
-// registers at 65536 / (128 * 7) = 73, i.e. 28 warps per SM instead of 12
-// at its natural ~155 registers; the traversal is latency-bound, so the
-// occupancy is worth the spilled values (measured faster on the sky-lit
-// 2.6M-triangle scene than 5 or 6)
-#ifndef NB_MEGA_MIN_BLOCKS
-#define NB_MEGA_MIN_BLOCKS 7
-#endif
-
-template <int ISECT, int FILM, bool EXT, bool DIFF = false>
-__global__ void __launch_bounds__(kMegaBlock, NB_MEGA_MIN_BLOCKS) megakernel(DevScene S, DevCamera C, MegaArgs a) {
-    extern __shared__ uint32_t smem[];
-    const uint32_t npix = C.w * C.h;
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t pix = idx % npix;
-    const uint32_t chunk = idx / npix;
-    RayStats rs{0u, 0u};
-    uint32_t paths = 0;
-    if (chunk < a.chunks) {
-        const uint32_t per = (a.nframes + a.chunks - 1) / a.chunks;
-        const uint32_t fb = chunk * per;
-        const uint32_t fe = min(fb + per, a.nframes);
-        SmemStack st{smem + threadIdx.x, (int)blockDim.x, S.stack_cap};
-        const uint32_t x = pix % C.w, y = pix / C.w;
-        float3 sum = f3(0.0f), comp = f3(0.0f);
-        float4 mean = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-        if (a.chunks == 1u && !a.fresh) {
-            if (FILM == NOOR_FILM_KAHAN) {
-                sum = f3(a.film_sum[pix]);
-                comp = f3(a.film_comp[pix]);
-            } else {
-                mean = a.film_sum[pix];
-            }
-        }
-        float3 hitp = f3(0.0f);
-        bool hit_valid = false;
-        const bool want_hit = (pix == C.center) && (chunk == a.chunks - 1u);
-        for (uint32_t f = fb; f < fe; ++f) {
-            const uint32_t frame = a.frame0 + f;
-            Rng rng{tea16(pix, frame)};
-            float3 o, d;
-            RayDiff rd{};
-            if (DIFF)
-                camera_ray_diff(C, x, y, rng, o, d, rd);
-            else
-                camera_ray<EXT>(C, x, y, rng, o, d);
-            hit_valid = false;
-            const float3 L = path_radiance<ISECT, EXT, DIFF>(S, o, d, rng, st, a.status, rs,
-                                                             want_hit ? &hitp : nullptr, &hit_valid, rd);
-            ++paths;
-            if (FILM == NOOR_FILM_KAHAN) {
-                kahan_add(sum, comp, L);
-            } else {
-                // framebuffer.set: lerp(old, new, 1/frame) (framebuffer.cuh:72-76)
-                const float4 old = frame > 1u ? mean : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-                const float t = 1.0f / (float)frame;
-                mean = make_float4(old.x + t * (L.x - old.x), old.y + t * (L.y - old.y), old.z + t * (L.z - old.z),
-                                   old.w + t * (1.0f - old.w));
-            }
-        }
-        if (a.chunks == 1u) {
-            if (FILM == NOOR_FILM_KAHAN) {
-                a.film_sum[pix] = make_float4(sum.x, sum.y, sum.z, 1.0f);
-                a.film_comp[pix] = make_float4(comp.x, comp.y, comp.z, 0.0f);
-            } else {
-                a.film_sum[pix] = mean;
-            }
-        } else {
-            const size_t o = (size_t)chunk * npix + pix;
-            a.part_sum[o] = make_float4(sum.x, sum.y, sum.z, 0.0f);
-            a.part_comp[o] = make_float4(comp.x, comp.y, comp.z, 0.0f);
-        }
-        if (want_hit) *a.lookat = make_float4(hitp.x, hitp.y, hitp.z, hit_valid ? 1.0f : 0.0f);
-    }
-    warp_count(a.counters + 0, rs.ext);
-    warp_count(a.counters + 1, rs.shadow);
-    warp_count(a.counters + 2, paths);
 }
 
 // folds the per-chunk partial sums into the Kahan film in chunk order
@@ -308,42 +221,11 @@ __global__ void k_debug_skydome(DevScene S, DevCamera C, uint32_t frame, float4*
 }
 
 // ------------------------------------------------------------ launchers
-static size_t stack_bytes(const DevScene& S, int block) { return (size_t)S.stack_cap * block * sizeof(uint32_t); }
-
 cudaError_t launch_megakernel(const DevScene& S, const DevCamera& C, const MegaArgs& a, cudaStream_t s) {
-    const uint32_t npix = C.w * C.h;
-    const uint64_t threads = (uint64_t)npix * a.chunks;
-    const uint32_t grid = (uint32_t)((threads + kMegaBlock - 1) / kMegaBlock);
-    const size_t sm = stack_bytes(S, kMegaBlock);
-    cudaError_t e;
-    // scenes without the extra lobes and lights, seen through a pinhole, run
-    // a specialisation without the other code (the kernel's registers are
-    // capped, so unused branches cost spills)
-    const bool ext_cam = C.type != NOOR_CAMERA_PERSP || C.lens_radius > 0.0f;
-#define NB_MK2(I, F, X, D)                                                                      \
-    do {                                                                                        \
-        e = cudaFuncSetAttribute(megakernel<I, F, X, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-        if (e != cudaSuccess) return e;                                                         \
-        megakernel<I, F, X, D><<<grid, kMegaBlock, sm, s>>>(S, C, a);                           \
-    } while (0)
-#define NB_MK(I, F)                     \
-    do {                                \
-        if (S.has_bump) NB_MK2(I, F, true, true); \
-        else if (S.ext_lobes || S.ext_lights || S.env_ref || S.has_tex || ext_cam) NB_MK2(I, F, true, false); \
-        else NB_MK2(I, F, false, false); \
-    } while (0)
-    if (S.isect == NOOR_ISECT_WATERTIGHT) {
-        if (S.film_mode == NOOR_FILM_KAHAN) NB_MK(NOOR_ISECT_WATERTIGHT, NOOR_FILM_KAHAN);
-        else NB_MK(NOOR_ISECT_WATERTIGHT, NOOR_FILM_REF_LERP);
-    } else {
-        if (S.film_mode == NOOR_FILM_KAHAN) NB_MK(NOOR_ISECT_REF_WALD, NOOR_FILM_KAHAN);
-        else NB_MK(NOOR_ISECT_REF_WALD, NOOR_FILM_REF_LERP);
-    }
-#undef NB_MK
-#undef NB_MK2
-    e = cudaGetLastError();
+    cudaError_t e = S.isect == NOOR_ISECT_WATERTIGHT ? launch_megakernel_wt(S, C, a, s) : launch_megakernel_wald(S, C, a, s);
     if (e != cudaSuccess) return e;
     if (a.chunks > 1u) {
+        const uint32_t npix = C.w * C.h;
         fold_partials<<<(npix + 255) / 256, 256, 0, s>>>(npix, a.chunks, a.fresh, a.film_sum, a.film_comp,
                                                           a.part_sum, a.part_comp);
         e = cudaGetLastError();

@@ -22,6 +22,9 @@ struct MegaArgs {
 };
 
 cudaError_t launch_megakernel(const DevScene& S, const DevCamera& C, const MegaArgs& a, cudaStream_t s);
+// ... its render kernel, per intersector
+cudaError_t launch_megakernel_wt(const DevScene& S, const DevCamera& C, const MegaArgs& a, cudaStream_t s);
+cudaError_t launch_megakernel_wald(const DevScene& S, const DevCamera& C, const MegaArgs& a, cudaStream_t s);
 cudaError_t launch_resolve(uint32_t npix, int mode, float inv_count, const float4* film_sum, float4* out,
                            cudaStream_t s);
 cudaError_t launch_trace_closest(const DevScene& S, const noor_ray* rays, noor_hit* hits, size_t n, uint32_t* status,

@@ -1,0 +1,361 @@
+// Staged rendering of cuda_path_tracer / noor_render_frames: the megakernel's
+// path loop cut into one launch per stage and bounce over every path of a
+// batch of frames, so that traversal runs without the shading code's
+// registers and shading runs over queues of one material kind.
+//
+//   begin    camera rays
+//   per bounce:
+//     extend  closest hit for the bounce's paths; surface hits are queued by
+//             material kind
+//     shade   one launch per kind: the direct light of the last bounce folded
+//             into the path's radiance, light (and MIS) samples whose shadow
+//             rays are queued, scatter, Russian roulette, the next ray
+//     shadow  any hit; blocked contributions are cancelled
+//   finish   what is pending and the sky or emitter a path ended on
+//   fold     each pixel's samples into the film, in frame order and with the
+//            megakernel's split into chunks
+//
+// Every path draws the megakernel's random numbers and evaluates the
+// megakernel's expressions in its order and with its rounding, so the film is
+// the megakernel's to the bit.  The megakernel is bound by divergence (8-10 of
+// 32 lanes: a warp runs until its longest path ends) and by instruction fetch;
+// the stages run 13 and more lanes of small kernels.  Measured against the
+// megakernel: 256x256 room 0.305 -> 0.255 ms, 1920x1080 of a 2.6M-triangle
+// sky scene 3.69 -> 2.39, sixteen 960x540 frames of an environment-lit field
+// 14.7 -> 4.1, four 641x359 frames of the textured room 4.02 -> 1.02.  The
+// extension of the next bounce runs beside the shadow rays in one launch: the
+// room's frame took 0.319 ms with a launch each.
+#pragma once
+#include "integrator.cuh"
+#include "kernels.h"
+
+namespace nb {
+
+constexpr int kStageKinds = 3;  // shade_kind: Lambert, conductor, the rest
+
+// counters of one bounce
+enum : int {
+    kStActive = kStageKinds,        // paths the bounce extends
+    kStShadow = kStageKinds + 1,    // shadow rays queued
+    kStTake = kStageKinds + 2,      // active paths taken by extend's warps
+    kStTakeShadow = kStageKinds + 3,
+    kStWords = 8
+};
+
+// how a path ended, beside the material types (hit2.y): nothing to add, or an
+// escape to a sky it counts
+constexpr uint32_t kStDone = 0x80000000u, kStSky = 0x40000000u;
+
+struct StageDev {
+    float4* o;          // origin
+    float4* d;          // direction, w = 1 after a specular bounce
+    float4* beta;       // throughput, w = 1 while contributions are pending
+    float4* L;          // radiance, w = RNG state bits
+    float4* pend;       // 2 per path: direct-light contribution, w = 1 while it counts
+    float4* pbeta;      // the throughput it is weighted by
+    float4* hit;        // t, u, v, triangle bits
+    uint2* hit2;        // instance, material type or kSt*
+    float4* diff;       // 4 per path where the scene has bump maps: the ray's differentials
+    uint32_t* queue[2]; // paths of this bounce and of the next (bounce 0: all)
+    uint32_t* qshade;   // kStageKinds * cap
+    uint32_t* qshadow;  // 2 * cap: path << 1 | which
+    float4* sh_o;       // origin, tmax
+    float4* sh_d;
+    uint32_t* count;    // kStWords per bounce, then one more
+    float4* first;      // per frame of the batch: the centre pixel's first hit (w = 1)
+    uint32_t* status;
+    unsigned long long* counters;   // [ext rays, shadow rays, paths]
+    uint32_t cap;       // queue stride
+    uint32_t paths;     // paths of the batch
+    uint32_t frames;    // frames of the batch
+    uint32_t frame0;    // number of its first frame
+};
+
+struct StageFold {
+    uint32_t first;     // index of the batch's first frame in the call
+    uint32_t total;     // frames of the call
+    uint32_t chunks;
+    uint32_t frame0;    // number of the call's first frame
+    uint32_t fresh;
+    int film_mode;
+    float4* film_sum;
+    float4* film_comp;
+    float4* part_sum;   // the running chunk's sum and compensation (chunks > 1)
+    float4* part_comp;
+    float4* lookat;
+};
+
+// pixel of the q-th pixel slot: 8x4 tiles in row-major order, row-major inside
+// a tile, so that a warp's camera rays form a compact bundle; pixels outside
+// the whole tiles follow row by row (the right strip, then the bottom rows)
+NB_D uint32_t stage_pixel(uint32_t q, uint32_t w, uint32_t h) {
+    const uint32_t w8 = w & ~7u, h4 = h & ~3u;
+    const uint32_t full = w8 * h4;
+    if (q < full) {
+        const uint32_t t = q >> 5, r = q & 31u;
+        const uint32_t tx = t % (w8 >> 3), ty = t / (w8 >> 3);
+        return (ty * 4u + (r >> 3)) * w + tx * 8u + (r & 7u);
+    }
+    q -= full;
+    const uint32_t rw = w - w8;
+    if (q < rw * h4) return (q / rw) * w + w8 + q % rw;
+    q -= rw * h4;
+    return (h4 + q / w) * w + q % w;
+}
+
+// warp-aggregated push: lanes of one warp may push onto different queues
+NB_D uint32_t stage_push(uint32_t* counter) {
+    const uint32_t active = __activemask();
+    const uint32_t peers = __match_any_sync(active, reinterpret_cast<unsigned long long>(counter));
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(peers) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(peers));
+    base = __shfl_sync(active, base, leader);
+    return base + __popc(peers & ((1u << lane) - 1u));
+}
+
+NB_D void stage_store_diff(const StageDev& W, uint32_t i, const RayDiff& r) {
+    W.diff[4 * i] = make_float4(r.odx.x, r.odx.y, r.odx.z, r.on ? 1.0f : 0.0f);
+    W.diff[4 * i + 1] = make_float4(r.ody.x, r.ody.y, r.ody.z, 0.0f);
+    W.diff[4 * i + 2] = make_float4(r.ddx.x, r.ddx.y, r.ddx.z, 0.0f);
+    W.diff[4 * i + 3] = make_float4(r.ddy.x, r.ddy.y, r.ddy.z, 0.0f);
+}
+NB_D RayDiff stage_load_diff(const StageDev& W, uint32_t i) {
+    const float4 a = W.diff[4 * i], b = W.diff[4 * i + 1], c = W.diff[4 * i + 2], e = W.diff[4 * i + 3];
+    RayDiff r;
+    r.on = a.w != 0.0f;
+    r.odx = f3(a);
+    r.ody = f3(b);
+    r.ddx = f3(c);
+    r.ddy = f3(e);
+    return r;
+}
+
+// path i: pixel slot i / frames, frame i % frames (all samples of a pixel side by side)
+template <bool EXT, bool DIFF>
+__global__ void __launch_bounds__(256) st_begin(DevCamera C, StageDev W) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= W.paths) return;
+    const uint32_t pix = stage_pixel(i / W.frames, C.w, C.h);
+    Rng rng{tea16(pix, W.frame0 + i % W.frames)};
+    float3 o, d;
+    if (DIFF) {
+        RayDiff rd{};
+        camera_ray_diff(C, pix % C.w, pix / C.w, rng, o, d, rd);
+        stage_store_diff(W, i, rd);
+    } else {
+        camera_ray<EXT>(C, pix % C.w, pix / C.w, rng, o, d);
+    }
+    W.o[i] = make_float4(o.x, o.y, o.z, 0.0f);
+    W.d[i] = make_float4(d.x, d.y, d.z, 0.0f);
+    W.beta[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    W.L[i] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(rng.s));
+    W.hit2[i] = make_uint2(0u, kStDone);
+}
+
+template <int ISECT, bool EXT>
+NB_D void stage_extend(const DevScene& S, const DevCamera& C, const StageDev& W, uint32_t bounce, const SmemStack& stk) {
+    uint32_t* cnt = W.count + bounce * kStWords;
+    const uint32_t n = bounce ? cnt[kStActive] : W.paths;
+    const uint32_t* queue = W.queue[bounce & 1u];
+    const uint32_t lane = threadIdx.x & 31, take = rays_per_warp(n);
+    for (;;) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(cnt + kStTake, take);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= n) break;
+        if (lane >= take || base + lane >= n) continue;
+        const uint32_t i = bounce ? queue[base + lane] : base + lane;
+        float tmax = kInf;
+        HitRec rec{0.0f, 0.0f, 0u, 0u, 0u};
+        const StoredRay ray{W.o + i, W.d + i};
+        const bool binary = S.mega4 == 0u;
+        if (!trace_closest4<ISECT, EXT>(S, ray, tmax, rec, stk, binary ? S.stack_cap : S.stack_cap4, binary, W.status)) {
+            const bool sky = S.sky_on && (bounce == 0 || W.d[i].w != 0.0f);
+            W.hit2[i] = make_uint2(0u, sky ? kStSky : kStDone);
+            continue;
+        }
+        W.hit[i] = make_float4(tmax, rec.u, rec.v, __uint_as_float(rec.tri));
+        uint32_t kind = rec.mtype;
+        if (rec.mtype & kEmitterMat)
+            // an emitter met by a bounce that does not count it adds nothing
+            kind = bounce == 0 || W.d[i].w != 0.0f ? rec.mtype : kStDone;
+        else
+            W.qshade[shade_kind(lobe_of(rec.mtype)) * W.cap + stage_push(cnt + shade_kind(lobe_of(rec.mtype)))] = i;
+        W.hit2[i] = make_uint2(rec.ins, kind);
+        if (bounce == 0 && stage_pixel(i / W.frames, C.w, C.h) == C.center) {
+            const float4 o = W.o[i], d = W.d[i];
+            W.first[i % W.frames] = make_float4(fmaf(tmax, d.x, o.x), fmaf(tmax, d.y, o.y), fmaf(tmax, d.z, o.z), 1.0f);
+        }
+    }
+}
+
+NB_D void stage_shadow(const StageDev& W, uint32_t* cnt, uint32_t i, uint32_t which, const ShadowRay& sr) {
+    const uint32_t k = stage_push(cnt + kStShadow);
+    W.qshadow[k] = (i << 1) | which;
+    W.sh_o[k] = make_float4(sr.o.x, sr.o.y, sr.o.z, sr.tmax);
+    W.sh_d[k] = make_float4(sr.d.x, sr.d.y, sr.d.z, 0.0f);
+}
+
+// the last bounce's direct light, as the megakernel adds it: L += beta * (c0 + c1)
+NB_D void stage_pending(const StageDev& W, uint32_t i, float3& L) {
+    const float4 p0 = W.pend[2 * i], p1 = W.pend[2 * i + 1], b = W.pbeta[i];
+    float3 Ld = p0.w != 0.0f ? f3(p0) : f3(0.0f);
+    if (p1.w != 0.0f) Ld += f3(p1);
+    L += f3(b) * Ld;
+}
+
+// One row of blocks per material kind (blockIdx.y), so that a short queue
+// shades beside a long one
+// Bound by latency and by instruction fetch at these sizes: 4, 6 or 8 blocks
+// per SM (16 to 32 warps) measure the same (1.10, 1.07, 1.09 ms for four
+// 641x359 frames of the textured room); 6 leaves 80 registers.
+template <int ISECT, bool EXT, bool DIFF>
+__global__ void __launch_bounds__(128, EXT ? 4 : 6) st_shade(DevScene S, StageDev W, uint32_t bounce) {
+    const uint32_t kind_q = blockIdx.y;
+    uint32_t* cnt = W.count + bounce * kStWords;
+    const uint32_t n = cnt[kind_q];
+    uint32_t* next = W.queue[(bounce & 1u) ^ 1u];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const uint32_t i = W.qshade[kind_q * W.cap + k];
+        const float4 ow = W.o[i], dw = W.d[i], bw = W.beta[i], Lw = W.L[i], hw = W.hit[i];
+        const uint2 h2 = W.hit2[i];
+        float3 L = f3(Lw), beta = f3(bw);
+        if (bw.w != 0.0f) stage_pending(W, i, L);
+        const float3 o = f3(ow), d = f3(dw);
+        HitRec rec{hw.y, hw.z, __float_as_uint(hw.w), h2.x, h2.y};
+        Isect I;
+        TangentOut to;
+        const bool tex = EXT && S.has_tex;
+        make_isect<ISECT, EXT, true>(S, o, d, hw.x, rec, I, tex ? &to : nullptr);
+        DevMaterial m = S.materials[I.mat];
+        RayDiff rd{};
+        HitDiff hd;
+        if (DIFF) {
+            rd = stage_load_diff(W, i);
+            if (rd.on) {
+                hd = hit_differential(I, to, rd);
+                if (I.mtype & NOOR_BUMP) bump(S, I.mat, I.uv, hd, I.F);
+            }
+        }
+        if (tex && m.tex_mask) apply_textures(S, I.mat, I.uv, m);
+        Rng rng{__float_as_uint(Lw.w)};
+        int li = 0;
+        bool picked;
+        ShadowRay sr;
+        const float3 c0 = light_sample_contrib<EXT>(S, m, I, rng, S.mis != 0, li, picked, sr);
+        const bool has0 = !is_black(c0);
+        if (has0) stage_shadow(W, cnt, i, 0, sr);
+        float3 c1 = f3(0.0f);
+        bool has1 = false;
+        if (S.mis && picked) {
+            c1 = bsdf_mis_contrib<EXT>(S, m, I, rng, li, sr);
+            has1 = !is_black(c1);
+            if (has1) stage_shadow(W, cnt, i, 1, sr);
+        }
+        if (has0 || has1) {
+            W.pend[2 * i] = make_float4(c0.x, c0.y, c0.z, has0 ? 1.0f : 0.0f);
+            W.pend[2 * i + 1] = make_float4(c1.x, c1.y, c1.z, has1 ? 1.0f : 0.0f);
+            W.pbeta[i] = make_float4(beta.x, beta.y, beta.z, 0.0f);
+        }
+        rng.next();
+        rng.next();
+        float3 wi;
+        float pdf;
+        uint32_t stype;
+        const float3 f = bsdf_sample<EXT>(I.lobe, m, I.F, I.wo, BSDF_ALL, rng, wi, pdf, stype);
+        bool alive = pdf != 0.0f;
+        if (alive) {
+            beta *= (is_catcher<EXT>(I) ? f * catcher_sky<EXT>(S, I) : f) * absdot(wi, I.F.n) / pdf;
+            if (!(I.mtype & kTransparentMat) && dot(wi, I.F.ng) < 0.0f) {
+                alive = false;
+            } else if (bounce >= S.rr) {
+                const float q = fmaxf(0.05f, 1.0f - maxcomp(beta));
+                if (rng.next() < q)
+                    alive = false;
+                else
+                    beta /= 1.0f - q;
+            }
+        }
+        if (alive) {
+            const float3 no = spawn_origin(I, wi, S.bias);
+            if (DIFF) {
+                RayDiff nd{};
+                if (rd.on && (I.mtype & kGlossyMat))
+                    nd = spawn_diff(I, hd, rd, no, wi, (I.mtype & kDielectricMat) ? m.coat_ior : 1.0f);
+                stage_store_diff(W, i, nd);
+            }
+            W.o[i] = make_float4(no.x, no.y, no.z, 0.0f);
+            W.d[i] = make_float4(wi.x, wi.y, wi.z, (I.mtype & kSpecularMat) ? 1.0f : 0.0f);
+            if (bounce + 1u < S.bounces) next[stage_push(cnt + kStWords + kStActive)] = i;
+        }
+        W.beta[i] = make_float4(beta.x, beta.y, beta.z, has0 || has1 ? 1.0f : 0.0f);
+        W.L[i] = make_float4(L.x, L.y, L.z, __uint_as_float(rng.s));
+        W.hit2[i].y = kStDone;
+    }
+}
+
+template <int ISECT, bool EXT>
+NB_D void stage_occlude(const DevScene& S, const StageDev& W, uint32_t bounce, const SmemStack& stk) {
+    uint32_t* cnt = W.count + bounce * kStWords;
+    const uint32_t n = cnt[kStShadow];
+    const uint32_t lane = threadIdx.x & 31, take = rays_per_warp(n);
+    for (;;) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(cnt + kStTakeShadow, take);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= n) break;
+        const uint32_t q = base + lane;
+        if (lane >= take || q >= n) continue;
+        const StoredRay ray{W.sh_o + q, W.sh_d + q};
+        const bool binary = S.mega4 == 0u;
+        if (trace_any4<ISECT, EXT>(S, ray, W.sh_o[q].w, stk, binary ? S.stack_cap : S.stack_cap4, binary, W.status))
+            W.pend[W.qshadow[q]].w = 0.0f;
+    }
+}
+
+// The rays of a shade step: the next bounce's extension (blockIdx.y 0) beside
+// the shadow rays (blockIdx.y 1), which only the next shade step waits for.
+// bounce: the shade step's; extend only before the first (bounce -1) and
+// shadow only after the last.
+template <int ISECT, bool EXT>
+__global__ void __launch_bounds__(128, 7) st_trace(DevScene S, DevCamera C, StageDev W, int bounce) {
+    extern __shared__ uint32_t smem[];
+    const SmemStack stk{smem + threadIdx.x, (int)blockDim.x, S.stack_cap};
+    if (blockIdx.y == 0) {
+        if (bounce + 1 < (int)S.bounces) stage_extend<ISECT, EXT>(S, C, W, (uint32_t)(bounce + 1), stk);
+    } else {
+        stage_occlude<ISECT, EXT>(S, W, (uint32_t)bounce, stk);
+    }
+}
+
+// what a path's radiance still lacks; the clamped radiance into L
+template <int ISECT, bool EXT>
+__global__ void __launch_bounds__(256) st_finish(DevScene S, StageDev W) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= W.paths) return;
+    const float4 Lw = W.L[i], bw = W.beta[i];
+    const uint2 h2 = W.hit2[i];
+    float3 L = f3(Lw);
+    const float3 beta = f3(bw);
+    if (bw.w != 0.0f) stage_pending(W, i, L);
+    if (h2.y == kStSky) {
+        L += beta * env_eval<EXT>(S, f3(W.d[i]) * rsqrtf(stage_length2(f3(W.d[i]))));
+    } else if (!(h2.y & kStDone)) {
+        if (h2.y & NOOR_MESHLIGHT) {
+            L += beta * area_le<EXT>(S.area_lights[h2.x], f3(W.d[i]));
+        } else if (h2.y & kEmitterMat) {
+            const float4 hw = W.hit[i];
+            const uint32_t tri = __float_as_uint(hw.w);
+            const uint32_t mi = ISECT == NOOR_ISECT_WATERTIGHT ? __ldg(&S.wtri[tri].attr).w : __ldg(&S.wald[tri].attr).w;
+            DevMaterial em = S.materials[mi];
+            if (EXT && S.has_tex && em.tex_mask) apply_textures(S, mi, f2(hw.y, hw.z), em);
+            L += beta * (em.emitter_scale * em.emittance);
+        }
+    }
+    L = clamp3(L, 0.0f, 100.0f);
+    W.L[i] = make_float4(L.x, L.y, L.z, 0.0f);
+}
+
+}  // namespace nb

@@ -76,6 +76,8 @@ struct Context {
     void* scratch = nullptr;
     void* adj_buf = nullptr;  // adjoint: per-sample radiance of one chunk + the forward's Kahan state
     size_t adj_bytes = 0;
+    void* stage_buf = nullptr;  // staged renderer: a batch's paths and queues
+    size_t stage_bytes = 0;
     cudaEvent_t events[8] = {};
     uint64_t launches = 0;
     WavefrontState* wf = nullptr;
@@ -87,6 +89,7 @@ int cuda_fail(cudaError_t e, const char* what);
 int need_ctx(Context*& C);
 int sync_and_check(Context& C, const char* what);
 int render_frames(Context& C, uint32_t frame0, uint32_t n);
+int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done);  // path_stages.cu
 void wavefront_release(Context& C);
 void noalloc_forget(int device);  // noalloc.cu
 

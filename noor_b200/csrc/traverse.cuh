@@ -982,4 +982,31 @@ NB_D bool trace_shadow(const DevScene& S, const World& world, float tmax, const 
     return trace_any<ISECT, EXT>(S, o, d, tmax, st, status);
 }
 
+// Rays a warp of this launch takes at a time from a list of n: 32, or fewer
+// where there are more warps than that makes work for -- the lanes of a warp
+// walk one after the other where their walks part, so a short list is spread
+// over the warps (150 us of extension for a few hundred scattered rays 32 to
+// a warp, the last bounces of a 1920x1080 frame, take 20 one to a warp)
+NB_D uint32_t rays_per_warp(uint32_t n) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    return min(32u, max(1u, (n + warps - 1u) / warps));
+}
+
+// The walks of the adjoint: the four-wide tree where the
+// scene has one and the binary walk's stack fits its capacity (else the binary
+// tree, whose stack overflow is reported at that capacity)
+template <int ISECT, bool EXT>
+NB_D bool path_closest(const DevScene& S, const float3& o, const float3& d, float& tmax, HitRec& rec,
+                       const SmemStack& st, uint32_t* status) {
+    const bool binary = S.mega4 == 0u;
+    return trace_closest4<ISECT, EXT>(S, HeldRay{o, d}, tmax, rec, st, binary ? S.stack_cap : S.stack_cap4, binary,
+                                      status);
+}
+template <int ISECT, bool EXT>
+NB_D bool path_any(const DevScene& S, const float3& o, const float3& d, float tmax, const SmemStack& st,
+                   uint32_t* status) {
+    const bool binary = S.mega4 == 0u;
+    return trace_any4<ISECT, EXT>(S, HeldRay{o, d}, tmax, st, binary ? S.stack_cap : S.stack_cap4, binary, status);
+}
+
 }  // namespace nb

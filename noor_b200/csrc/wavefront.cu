@@ -512,14 +512,14 @@ __global__ void __launch_bounds__(NB_TRAV_THREADS, WIDE ? NB_TRAV_MIN_BLOCKS_WID
         // camera rays: the work items regen took this iteration
         const unsigned long long wn = W.work_next[0] < W.total ? W.work_next[0] : W.total;
         const uint32_t nc = (uint32_t)(wn - W.work_next[1]), n = W.counters[kCntActive];
-        const uint32_t lane = threadIdx.x & 31;
+        const uint32_t lane = threadIdx.x & 31, take = rays_per_warp(n);
         for (;;) {
             uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(W.counters + kCntTakeExt, 32u);
+            if (lane == 0) base = atomicAdd(W.counters + kCntTakeExt, take);
             base = __shfl_sync(0xFFFFFFFFu, base, 0);
             if (base >= n) break;
             const uint32_t i = base + lane;
-            if (i >= n) continue;
+            if (lane >= take || i >= n) continue;
             extend_slot<ISECT, MULTI, EXT, WIDE>(W, S1, i < nc ? W.ext_perm[i] : W.ext_perm[W.cap + (i - nc)], stk);
         }
         return;
@@ -715,14 +715,14 @@ __global__ void __launch_bounds__(NB_TRAV_THREADS, WIDE ? NB_TRAV_MIN_BLOCKS_WID
     SmemStack stk{smem + threadIdx.x, (int)blockDim.x, W.stack_cap};
 
 #if NB_SHADOW_FETCH
-    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31, take = rays_per_warp(n);
     for (;;) {
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(W.counters + kCntTake, 32u);
+        if (lane == 0) base = atomicAdd(W.counters + kCntTake, take);
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
         if (base >= n) break;
         const uint32_t i = base + lane;
-        if (i >= n) continue;
+        if (lane >= take || i >= n) continue;
 #else
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 #endif

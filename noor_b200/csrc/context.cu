@@ -286,7 +286,7 @@ int build_distribution(Context& C, SceneState& st) {
     EnvBuild& b = st.env;
     cudaError_t e;
     if (st.sky_type == NOOR_SKY_PHYSICAL)
-        e = launch_env_func_from_sky(st.dev.hosek, b.w, b.h, b.func, C.stream);
+        e = launch_env_func_from_sky(st.dev.hosek, b.w, b.h, b.scratch, b.func, C.stream);
     else
         e = launch_env_func_from_texture(st.dev.env, b.w, b.h, b.func, C.stream);
     if (e != cudaSuccess) return cuda_fail(e, "env func");

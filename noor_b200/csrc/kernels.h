@@ -53,8 +53,9 @@ struct EnvBuild {
 };
 // func from the env texels (luminance x sin(theta) per texel)
 cudaError_t launch_env_func_from_texture(const float4* env, int w, int h, float* func, cudaStream_t s);
-// func from the Hosek sky (4x4 supersampled luminance x sin(theta) per cell)
-cudaError_t launch_env_func_from_sky(const DevHosek& H, int w, int h, float* func, cudaStream_t s);
+// func from the Hosek sky (4x4 supersampled luminance x sin(theta) per cell);
+// scratch: room for 8 w doubles
+cudaError_t launch_env_func_from_sky(const DevHosek& H, int w, int h, double* scratch, float* func, cudaStream_t s);
 // FP64 row/marginal prefix sums -> normalised FP32 CDFs
 cudaError_t launch_env_cdf(const EnvBuild& b, cudaStream_t s);
 // NOOR_ENV_REFERENCE: the physical sky baked as sin(theta) x radiance into a

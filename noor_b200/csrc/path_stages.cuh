@@ -69,6 +69,7 @@ struct StageDev {
     uint32_t paths;     // paths of the batch
     uint32_t frames;    // frames of the batch
     uint32_t frame0;    // number of its first frame
+    uint32_t keep;      // paths between the pend and pbeta entries of one bounce and the next (0: reused)
 };
 
 struct StageFold {
@@ -191,11 +192,13 @@ NB_D void stage_extend(const DevScene& S, const DevCamera& C, const StageDev& W,
     }
 }
 
-NB_D void stage_shadow(const StageDev& W, uint32_t* cnt, uint32_t i, uint32_t which, const ShadowRay& sr) {
+// queues shadow ray `which` of path i; returns its place
+NB_D uint32_t stage_shadow(const StageDev& W, uint32_t* cnt, uint32_t i, uint32_t which, const ShadowRay& sr) {
     const uint32_t k = stage_push(cnt + kStShadow);
     W.qshadow[k] = (i << 1) | which;
     W.sh_o[k] = make_float4(sr.o.x, sr.o.y, sr.o.z, sr.tmax);
     W.sh_d[k] = make_float4(sr.d.x, sr.d.y, sr.d.z, 0.0f);
+    return k;
 }
 
 // the last bounce's direct light, as the megakernel adds it: L += beta * (c0 + c1)
@@ -311,7 +314,7 @@ NB_D void stage_occlude(const DevScene& S, const StageDev& W, uint32_t bounce, c
         const StoredRay ray{W.sh_o + q, W.sh_d + q};
         const bool binary = S.mega4 == 0u;
         if (trace_any4<ISECT, EXT>(S, ray, W.sh_o[q].w, stk, binary ? S.stack_cap : S.stack_cap4, binary, W.status))
-            W.pend[W.qshadow[q]].w = 0.0f;
+            W.pend[2u * (size_t)W.keep * bounce + W.qshadow[q]].w = 0.0f;
     }
 }
 

@@ -1,6 +1,8 @@
 // Render and parity kernels: the film fold, ray-batch traversal and the
 // device-routine evaluators used by the parity tests (the megakernel is in
 // megakernel.cuh).
+#include <type_traits>
+
 #include "kernels.h"
 #include "integrator.cuh"
 
@@ -40,8 +42,13 @@ __global__ void film_resolve(uint32_t npix, int mode, float inv_count, const flo
     out[pix] = mode == NOOR_FILM_KAHAN ? make_float4(s.x * inv_count, s.y * inv_count, s.z * inv_count, 1.0f) : s;
 }
 
-template <int ISECT, bool WIDE>
-__global__ void __launch_bounds__(kTraceBlock) k_trace_closest(DevScene S, const noor_ray* rays, noor_hit* hits,
+// EXT false: the scene has no sphere, disk or delta lights and no textures.
+// 7 blocks (72 registers) as the wavefront's walks: a million scattered rays
+// on 2.6M triangles, closest and any hit, take 0.556 ms (8 blocks 0.585, 6
+// 0.571, 5 0.579; 0.673 with the extra lights' code and no bound).
+constexpr int kTraceMinBlocks = 7;
+template <int ISECT, bool WIDE, bool EXT>
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_trace_closest(DevScene S, const noor_ray* rays, noor_hit* hits,
                                                                size_t n, uint32_t* status) {
     extern __shared__ uint32_t smem[];
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -51,7 +58,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_closest(DevScene S, const
     float tmax = r.tmax;
     HitRec rec{0.0f, 0.0f, 0u, 0u, 0u};
     const HeldRay world{f3(r.org[0], r.org[1], r.org[2]), f3(r.dir[0], r.dir[1], r.dir[2])};
-    const bool h = trace_primary<ISECT, true, WIDE>(S, world, tmax, rec, st, status);
+    const bool h = trace_primary<ISECT, EXT, WIDE>(S, world, tmax, rec, st, status);
     noor_hit o;
     o.t = tmax;
     o.tri_idx = rec.tri;
@@ -64,8 +71,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_closest(DevScene S, const
     hits[i] = o;
 }
 
-template <int ISECT, bool WIDE>
-__global__ void __launch_bounds__(kTraceBlock) k_trace_any(DevScene S, const noor_ray* rays, uint32_t* occ,
+template <int ISECT, bool WIDE, bool EXT>
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_trace_any(DevScene S, const noor_ray* rays, uint32_t* occ,
                                                            size_t n, uint32_t* status) {
     extern __shared__ uint32_t smem[];
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -73,7 +80,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_any(DevScene S, const noo
     SmemStack st{smem + threadIdx.x, (int)blockDim.x, S.stack_cap};
     const noor_ray r = rays[i];
     const HeldRay world{f3(r.org[0], r.org[1], r.org[2]), f3(r.dir[0], r.dir[1], r.dir[2])};
-    occ[i] = trace_shadow<ISECT, true, WIDE>(S, world, r.tmax, st, status) ? 1u : 0u;
+    occ[i] = trace_shadow<ISECT, EXT, WIDE>(S, world, r.tmax, st, status) ? 1u : 0u;
 }
 
 __global__ void k_camera_rays(DevCamera C, uint32_t frame, noor_ray* rays) {
@@ -240,8 +247,8 @@ cudaError_t launch_resolve(uint32_t npix, int mode, float inv_count, const float
 }
 
 // one launch of a ray-batch kernel: the four-wide or the binary traversal,
-// per intersector
-template <template <int, bool> class K, class T>
+// per intersector, with or without the extra lights' code
+template <template <int, bool, bool> class K, class T>
 static cudaError_t launch_trace(const DevScene& S, bool wide, const noor_ray* rays, T* out, size_t n,
                                 uint32_t* status, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
@@ -254,17 +261,22 @@ static cudaError_t launch_trace(const DevScene& S, bool wide, const noor_ray* ra
         kern<<<grid, kTraceBlock, sm, s>>>(S, rays, out, n, status);
         return cudaGetLastError();
     };
-    if (S.isect == NOOR_ISECT_WATERTIGHT)
-        return wide ? go(K<NOOR_ISECT_WATERTIGHT, true>::fn) : go(K<NOOR_ISECT_WATERTIGHT, false>::fn);
-    return wide ? go(K<NOOR_ISECT_REF_WALD, true>::fn) : go(K<NOOR_ISECT_REF_WALD, false>::fn);
+    const bool ext = S.ext_lights || S.has_tex;
+    auto pick = [&](auto isect) {
+        constexpr int I = decltype(isect)::value;
+        if (wide) return ext ? go(K<I, true, true>::fn) : go(K<I, true, false>::fn);
+        return ext ? go(K<I, false, true>::fn) : go(K<I, false, false>::fn);
+    };
+    if (S.isect == NOOR_ISECT_WATERTIGHT) return pick(std::integral_constant<int, NOOR_ISECT_WATERTIGHT>());
+    return pick(std::integral_constant<int, NOOR_ISECT_REF_WALD>());
 }
-template <int I, bool W>
+template <int I, bool W, bool X>
 struct ClosestK {
-    static constexpr auto fn = k_trace_closest<I, W>;
+    static constexpr auto fn = k_trace_closest<I, W, X>;
 };
-template <int I, bool W>
+template <int I, bool W, bool X>
 struct AnyK {
-    static constexpr auto fn = k_trace_any<I, W>;
+    static constexpr auto fn = k_trace_any<I, W, X>;
 };
 
 cudaError_t launch_trace_closest(const DevScene& S, const noor_ray* rays, noor_hit* hits, size_t n, uint32_t* status,

@@ -21,6 +21,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <exception>
+#include <thread>
 
 #include "bvh_gpu.h"
 #include "../../include/noor_b200.h"
@@ -286,6 +288,72 @@ __device__ bool write_inner(const Out& o, const Params& P, const Task& t, uint32
 }
 
 // ------------------------------------------------------------ kernels
+// Model::computeBBoxes (model.cpp:73-108): the box of each triangle, and the
+// box of each mesh's triangles and of their centroids as ordered keys (the
+// first of equal coordinates, as the host's loop keeps it).  One block per
+// run of kBoxRun triangles of one mesh: the keys meet in registers, then
+// over the warp, and once per warp in global memory.  Bound by the gather of
+// the vertices.  1.3M triangles take 4.2 ms with the upload of their indices
+// and vertices, which later steps read too; the host's loop took 12.5 ms, and
+// the upload of its boxes came on top.
+constexpr uint32_t kBoxRun = 2048;
+struct BoxRun {
+    uint32_t mesh, begin, end;  // triangles begin .. end - 1, mesh's first one is at `first`
+    uint32_t first;
+};
+__global__ void __launch_bounds__(256) k_boxes(const BoxRun* runs, const uint32_t* vi, const float4* vtx,
+                                               float* tri_box, uint32_t* order, unsigned long long* keys) {
+    const BoxRun r = runs[blockIdx.x];
+    unsigned long long k[kKeys];
+    keys_init(k);
+    for (uint32_t t = r.begin + threadIdx.x; t < r.end; t += blockDim.x) {
+        float v[3][3];
+        for (int j = 0; j < 3; ++j) {
+            const float4 p = vtx[vi[3 * (size_t)t + j]];
+            v[j][0] = p.x;
+            v[j][1] = p.y;
+            v[j][2] = p.z;
+        }
+        float tb[6], c[3];
+        for (int i = 0; i < 3; ++i) {
+            tb[i] = mn(mn(v[0][i], v[1][i]), v[2][i]);
+            tb[3 + i] = mx(mx(v[0][i], v[1][i]), v[2][i]);
+        }
+        centroid(tb, c);
+        for (int i = 0; i < 6; ++i) tri_box[6 * (size_t)t + i] = tb[i];
+        order[t] = t;
+        const uint32_t q = t - r.first;
+        for (int i = 0; i < 3; ++i) {
+            k[i] = min(k[i], kmin(tb[i], q));
+            k[3 + i] = max(k[3 + i], kmax(tb[3 + i], q));
+            k[6 + i] = min(k[6 + i], kmin(c[i], q));
+            k[9 + i] = max(k[9 + i], kmax(c[i], q));
+        }
+    }
+    for (int i = 0; i < kKeys; ++i) {
+        const bool lo = i < 3 || (i >= 6 && i < 9);
+        for (int d = 16; d > 0; d >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, k[i], d);
+            k[i] = lo ? min(k[i], o) : max(k[i], o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            if (lo)
+                atomicMin(keys + (size_t)r.mesh * kKeys + i, k[i]);
+            else
+                atomicMax(keys + (size_t)r.mesh * kKeys + i, k[i]);
+        }
+    }
+}
+__global__ void k_boxes_init(unsigned long long* keys, uint32_t n_meshes) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_meshes) keys_init(keys + (size_t)i * kKeys);
+}
+// box lo, box hi, centroid lo, centroid hi of each mesh that has triangles
+__global__ void k_boxes_decode(const unsigned long long* keys, uint32_t n_meshes, float* out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_meshes * kKeys) out[i] = kval(keys[i]);
+}
+
 // leaf tests of BVH::recursiveBuild that need no split search (level, count);
 // the rest go to the tiny / small / large lists
 __global__ void k_classify(const Task* tasks, uint32_t n, Params P, Out o, uint32_t* tiny, uint32_t* small,
@@ -733,22 +801,18 @@ __global__ void k_dfs(Rec* recs, const uint32_t* level_recs, uint32_t n) {
     recs[r.a].dfs = r.dfs + 1;
     recs[r.b].dfs = r.dfs + 1 + recs[r.a].size;
 }
-__global__ void k_write(const Rec* recs, uint32_t n_rec, const uint32_t* mesh_off, uint32_t* out) {
+// the payload's two node arrays, right-child words counted from the scene's
+// first node: what the host keeps is copied from here and not touched again
+__global__ void k_write(const Rec* recs, uint32_t n_rec, const uint32_t* mesh_off, uint4* lo, uint4* hi) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_rec) return;
     const Rec& r = recs[i];
-    uint32_t* w = out + 8 * ((size_t)mesh_off[r.mesh] + r.dfs);
-    for (int k = 0; k < 3; ++k) {
-        w[k] = __float_as_uint(r.box[k]);
-        w[4 + k] = __float_as_uint(r.box[3 + k]);
-    }
-    if (r.kind & kLeafBit) {
-        w[3] = r.a;
-        w[7] = NOOR_TRI_LEAF_MASK | r.b;
-    } else {
-        w[3] = recs[r.b].dfs;
-        w[7] = r.kind;
-    }
+    const uint32_t off = mesh_off[r.mesh];
+    const bool leaf = (r.kind & kLeafBit) != 0u;
+    lo[off + r.dfs] = make_uint4(__float_as_uint(r.box[0]), __float_as_uint(r.box[1]), __float_as_uint(r.box[2]),
+                                 leaf ? r.a : off + recs[r.b].dfs);
+    hi[off + r.dfs] = make_uint4(__float_as_uint(r.box[3]), __float_as_uint(r.box[4]), __float_as_uint(r.box[5]),
+                                 leaf ? NOOR_TRI_LEAF_MASK | r.b : r.kind);
 }
 
 
@@ -960,22 +1024,173 @@ static void keep_pool() {
 
 }  // namespace
 
-int gpu_build_blas(const float* tri_box, uint32_t n_tris, const std::vector<GpuMesh>& meshes, const GpuBvhParams& bp,
-                   std::vector<uint32_t>& tri_order, std::vector<GpuTree>& trees, double* device_ms,
-                   std::string& err) {
-    auto fail = [&](const char* what, cudaError_t e) {
-        err = std::string("GPU BVH build: ") + what + ": " + cudaGetErrorString(e);
-        return NOOR_ERR_CUDA;
-    };
-    const uint32_t M = (uint32_t)meshes.size();
-    trees.assign(M, GpuTree());
-    if (M == 0) return NOOR_OK;
-    if (bp.num_bins < 2 || bp.num_bins > kMaxBins) {
-        err = "GPU BVH build: num_bins must be in [2, 64]";
+// a host thread for copies from and to pageable memory, which hold up the
+// thread that issues them; where none can be had the caller does them itself
+struct SideThread {
+    std::thread t;
+    bool on = true;
+    template <class F>
+    void run(F f) {
+        join();
+        if (!on) return f();
+        try {
+            t = std::thread(f);
+        } catch (const std::exception&) {
+            f();
+        }
+    }
+    void join() {
+        if (t.joinable()) t.join();
+    }
+};
+
+// Scenes of fewer triangles are built without side threads and their streams:
+// starting them takes longer than their copies (320 triangles: 1.61 ms with
+// them, 1.49 without; 40960: 5.3 with them, 7.5 without)
+constexpr uint32_t kSideMinTris = 32768;
+
+struct GpuPayload::Impl {
+    GpuInput in;
+    GpuTailOut& out;
+    int dev = 0;
+    cudaStream_t s = nullptr, s2 = nullptr, s3 = nullptr;  // the steps', the side threads'
+    cudaEvent_t allocated = nullptr;
+    // of the side threads' copies: read after their join
+    cudaError_t up_error = cudaSuccess, down_error = cudaSuccess, down2_error = cudaSuccess;
+    bool ready = false;
+    SideThread side, side2;
+    DevBuf b_vi, b_vtx, b_ni, b_ui, b_nrm, b_uv, b_mi, b_box, b_order, b_lo, b_hi;
+    uint32_t *d_vi = nullptr, *d_ni = nullptr, *d_ui = nullptr, *d_mi = nullptr, *d_order = nullptr;
+    float4 *d_vtx = nullptr, *d_nrm = nullptr;
+    float2* d_uv = nullptr;
+    float* d_box = nullptr;
+    uint4 *d_lo = nullptr, *d_hi = nullptr;
+    size_t n_nodes = 0;
+
+    Impl(const GpuInput& i, GpuTailOut& o) : in(i), out(o) {}
+    ~Impl() {
+        side.join();
+        side2.join();
+        // the buffers are given back on s
+        if (s2) cudaStreamSynchronize(s2);
+        if (s3) cudaStreamSynchronize(s3);
+        for (DevBuf* b : {&b_vi, &b_vtx, &b_ni, &b_ui, &b_nrm, &b_uv, &b_mi, &b_box, &b_order, &b_lo, &b_hi})
+            if (b->p) {
+                cudaFreeAsync(b->p, s);
+                b->p = nullptr;
+            }
+        if (allocated) cudaEventDestroy(allocated);
+        if (s2 && s2 != s) cudaStreamDestroy(s2);
+        if (s3 && s3 != s) cudaStreamDestroy(s3);
+        if (s) cudaStreamDestroy(s);
+    }
+    // streams, the scene's buffers, and the uploads
+    cudaError_t open();
+};
+
+cudaError_t GpuPayload::Impl::open() {
+    const size_t T = in.n_tris, C = 3 * T;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) || (e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking))) return e;
+    side.on = side2.on = in.n_tris >= kSideMinTris;
+    if (!side.on)
+        s2 = s3 = s;
+    else if ((e = cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking)) ||
+             (e = cudaStreamCreateWithFlags(&s3, cudaStreamNonBlocking)))
+        return e;
+    if ((e = cudaEventCreateWithFlags(&allocated, cudaEventDisableTiming)))
+        return e;
+    keep_pool();
+    if ((e = dalloc(s, b_vi, C, &d_vi)) || (e = dalloc(s, b_ni, C, &d_ni)) || (e = dalloc(s, b_ui, C, &d_ui)) ||
+        (e = dalloc(s, b_vtx, in.n_vertices, &d_vtx)) || (e = dalloc(s, b_nrm, in.n_normals, &d_nrm)) ||
+        (e = dalloc(s, b_uv, in.n_uvs, &d_uv)) || (e = dalloc(s, b_mi, T, &d_mi)) ||
+        (e = dalloc(s, b_box, 6 * T, &d_box)) || (e = dalloc(s, b_order, T, &d_order)) ||
+        (e = cudaEventRecord(allocated, s)) || (e = cudaStreamWaitEvent(s2, allocated, 0)))
+        return e;
+    ready = true;
+    side.run([this, T, C]() {
+        cudaError_t r;
+        (r = cudaSetDevice(dev)) || (r = cudaMemcpyAsync(d_ni, in.nindices, 4 * C, cudaMemcpyHostToDevice, s2)) ||
+            (r = cudaMemcpyAsync(d_ui, in.uvindices, 4 * C, cudaMemcpyHostToDevice, s2)) ||
+            (r = cudaMemcpyAsync(d_nrm, in.normals, 16 * (size_t)in.n_normals, cudaMemcpyHostToDevice, s2)) ||
+            (r = cudaMemcpyAsync(d_uv, in.uvs, 8 * (size_t)in.n_uvs, cudaMemcpyHostToDevice, s2)) ||
+            (r = cudaMemcpyAsync(d_mi, in.material_indices, 4 * T, cudaMemcpyHostToDevice, s2)) ||
+            (r = cudaStreamSynchronize(s2));
+        up_error = r;
+    });
+    // one write per 4 KiB: the first one on a page gets it from the system
+    side2.run([this]() {
+        for (auto* w : {&out.wald[0], &out.wald[1], &out.wald[2], &out.attr})
+            for (size_t i = 0; i < w->size(); i += 1024) static_cast<volatile uint32_t*>(w->data())[i] = 0;
+    });
+    if ((e = cudaMemcpyAsync(d_vi, in.vindices, 4 * C, cudaMemcpyHostToDevice, s))) return e;
+    return cudaMemcpyAsync(d_vtx, in.vertices, 16 * (size_t)in.n_vertices, cudaMemcpyHostToDevice, s);
+}
+
+GpuPayload::GpuPayload(const GpuInput& in, GpuTailOut& out) : I(new Impl(in, out)) {}
+GpuPayload::~GpuPayload() = default;
+
+static int gpu_fail(std::string& err, const char* step, const char* what, cudaError_t e) {
+    err = std::string(step) + ": " + what + ": " + cudaGetErrorString(e);
+    return NOOR_ERR_CUDA;
+}
+
+int GpuPayload::boxes(std::vector<GpuMesh>& meshes, std::string& err) {
+    auto fail = [&](const char* what, cudaError_t e) { return gpu_fail(err, "GPU BVH build", what, e); };
+    if (I->in.n_tris >= 0x7fffffffu) {
+        err = "GPU BVH build: too many triangles";
         return NOOR_ERR_INVALID;
     }
-    if (n_tris >= 0x7fffffffu) {
-        err = "GPU BVH build: too many triangles";
+    cudaError_t e = I->open();
+    if (e != cudaSuccess) return fail("upload", e);
+    cudaStream_t s = I->s;
+    const uint32_t M = (uint32_t)meshes.size();
+    std::vector<BoxRun> runs;
+    for (uint32_t m = 0; m < M; ++m) {
+        const uint32_t b = meshes[m].start, n = meshes[m].count;
+        if ((size_t)b + n > I->in.n_tris) {
+            err = "GPU BVH build: mesh range outside the triangles";
+            return NOOR_ERR_INVALID;
+        }
+        for (uint32_t o = 0; o < n; o += kBoxRun) runs.push_back(BoxRun{m, b + o, b + std::min(n, o + kBoxRun), b});
+    }
+    DevBuf b_runs, b_keys, b_out;
+    BoxRun* d_runs;
+    unsigned long long* d_keys;
+    float* d_out;
+    std::vector<float> out((size_t)M * kKeys);
+    if ((e = dalloc(s, b_runs, runs.size(), &d_runs)) || (e = dalloc(s, b_keys, (size_t)M * kKeys, &d_keys)) ||
+        (e = dalloc(s, b_out, (size_t)M * kKeys, &d_out)) ||
+        (e = cudaMemcpyAsync(d_runs, runs.data(), sizeof(BoxRun) * runs.size(), cudaMemcpyHostToDevice, s)))
+        return fail("boxes", e);
+    k_boxes_init<<<(M + 255) / 256, 256, 0, s>>>(d_keys, M);
+    if (!runs.empty())
+        k_boxes<<<(uint32_t)runs.size(), 256, 0, s>>>(d_runs, I->d_vi, I->d_vtx, I->d_box, I->d_order, d_keys);
+    k_boxes_decode<<<(M * kKeys + 255) / 256, 256, 0, s>>>(d_keys, M, d_out);
+    if ((e = cudaGetLastError()) ||
+        (e = cudaMemcpyAsync(out.data(), d_out, 4 * out.size(), cudaMemcpyDeviceToHost, s)) ||
+        (e = cudaStreamSynchronize(s)))
+        return fail("boxes", e);
+    for (uint32_t m = 0; m < M; ++m) {
+        if (meshes[m].count == 0) continue;  // left as the caller's empty box
+        std::memcpy(meshes[m].box, out.data() + (size_t)m * kKeys, 24);
+        std::memcpy(meshes[m].cbox, out.data() + (size_t)m * kKeys + 6, 24);
+    }
+    return NOOR_OK;
+}
+
+int GpuPayload::trees(const std::vector<GpuMesh>& meshes, const GpuBvhParams& bp, const std::vector<uint32_t>& lead,
+                      uint32_t others, std::vector<GpuTree>& trees, double* device_ms, std::string& err) {
+    auto fail = [&](const char* what, cudaError_t e) { return gpu_fail(err, "GPU BVH build", what, e); };
+    const uint32_t n_tris = I->in.n_tris;
+    const uint32_t M = (uint32_t)meshes.size();
+    trees.assign(M, GpuTree());
+    if (!I->ready) {
+        err = "GPU BVH build: no boxes";
+        return NOOR_ERR_INVALID;
+    }
+    if (bp.num_bins < 2 || bp.num_bins > kMaxBins) {
+        err = "GPU BVH build: num_bins must be in [2, 64]";
         return NOOR_ERR_INVALID;
     }
     Params P;
@@ -995,23 +1210,18 @@ int gpu_build_blas(const float* tri_box, uint32_t n_tris, const std::vector<GpuM
     const size_t max_chunks = 2 * ((size_t)n_tris / kChunk) + M + 8;
     const size_t max_large = (size_t)n_tris / kSmallCap + M + 8;
 
-    cudaStream_t s;
-    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (e != cudaSuccess) return fail("stream", e);
-    struct StreamGuard {
-        cudaStream_t s;
-        ~StreamGuard() { cudaStreamDestroy(s); }
-    } sg{s};
-    keep_pool();
+    cudaStream_t s = I->s;
+    cudaError_t e;
     TimingEvents te;
     if ((e = te.create())) return fail("events", e);
     cudaEvent_t ev0 = te.a, ev1 = te.b;
 
-    DevBuf b_box, b_order, b_tmp, b_rank, b_sF, b_sT, b_pred, b_tasks0, b_tasks1, b_recs, b_levels, b_tiny, b_small,
-        b_large, b_ctl, b_stats, b_splits, b_chunks, b_c0, b_ctrue, b_cbefore, b_gkeys, b_gcnt, b_meshoff, b_out;
-    float* d_box;
-    uint32_t *d_order, *d_tmp, *d_rank, *d_sF, *d_sT, *d_levels, *d_tiny, *d_small, *d_large, *d_stats, *d_c0,
-        *d_ctrue, *d_cbefore, *d_gcnt, *d_meshoff, *d_out;
+    DevBuf b_tmp, b_rank, b_sF, b_sT, b_pred, b_tasks0, b_tasks1, b_recs, b_levels, b_tiny, b_small,
+        b_large, b_ctl, b_stats, b_splits, b_chunks, b_c0, b_ctrue, b_cbefore, b_gkeys, b_gcnt, b_meshoff;
+    const float* d_box = I->d_box;
+    uint32_t* d_order = I->d_order;
+    uint32_t *d_tmp, *d_rank, *d_sF, *d_sT, *d_levels, *d_tiny, *d_small, *d_large, *d_stats, *d_c0,
+        *d_ctrue, *d_cbefore, *d_gcnt, *d_meshoff;
     unsigned char* d_pred;
     Task *d_tasks[2];
     Rec* d_recs;
@@ -1020,7 +1230,7 @@ int gpu_build_blas(const float* tri_box, uint32_t n_tris, const std::vector<GpuM
     Chunk* d_chunks;
     unsigned long long* d_gkeys;
     const size_t N = n_tris;
-    if ((e = dalloc(s, b_box, 6 * N, &d_box)) || (e = dalloc(s, b_order, N, &d_order)) || (e = dalloc(s, b_tmp, N, &d_tmp)) ||
+    if ((e = dalloc(s, b_tmp, N, &d_tmp)) ||
         (e = dalloc(s, b_rank, N, &d_rank)) || (e = dalloc(s, b_sF, N, &d_sF)) || (e = dalloc(s, b_sT, N, &d_sT)) ||
         (e = dalloc(s, b_pred, N, &d_pred)) || (e = dalloc(s, b_tasks0, P.task_cap, &d_tasks[0])) ||
         (e = dalloc(s, b_tasks1, P.task_cap, &d_tasks[1])) || (e = dalloc(s, b_recs, P.cap, &d_recs)) ||
@@ -1058,15 +1268,9 @@ int gpu_build_blas(const float* tri_box, uint32_t n_tris, const std::vector<GpuM
         t.mesh = i;
         std::memcpy(t.box, meshes[i].box, 24);
         std::memcpy(t.cbox, meshes[i].cbox, 24);
-        if ((size_t)t.start + t.count > N) {
-            err = "GPU BVH build: mesh range outside the triangles";
-            return NOOR_ERR_INVALID;
-        }
     }
     cudaEventRecord(ev0, s);
-    if ((e = cudaMemcpyAsync(d_box, tri_box, 24 * N, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_order, tri_order.data(), 4 * N, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_tasks[0], roots.data(), sizeof(Task) * M, cudaMemcpyHostToDevice, s)) ||
+    if ((e = cudaMemcpyAsync(d_tasks[0], roots.data(), sizeof(Task) * M, cudaMemcpyHostToDevice, s)) ||
         (e = cudaMemsetAsync(d_stats, 0, 16 * (size_t)M, s)))
         return fail("upload", e);
     Ctl ctl{};
@@ -1175,33 +1379,33 @@ int gpu_build_blas(const float* tri_box, uint32_t n_tris, const std::vector<GpuM
         (e = cudaStreamSynchronize(s)))
         return fail("sizes", e);
     std::vector<uint32_t> mesh_off(M);
-    size_t total = 0;
+    size_t total = 0, before = 0;
     for (uint32_t i = 0; i < M; ++i) {
-        mesh_off[i] = (uint32_t)total;
-        total += root_recs[i].size;
+        mesh_off[i] = (uint32_t)total + lead[i];
+        total += lead[i] + root_recs[i].size;
+        trees[i].first = mesh_off[i];
+        before += lead[i];
     }
-    if (total != n_rec) {
+    if (total - before != n_rec || before > others) {
         err = "GPU BVH build: record count mismatch";
         return NOOR_ERR_CUDA;
     }
-    if ((e = dalloc(s, b_out, 8 * total, &d_out)) ||
+    I->n_nodes = (size_t)n_rec + others;
+    if ((e = dalloc(s, I->b_lo, I->n_nodes, &I->d_lo)) || (e = dalloc(s, I->b_hi, I->n_nodes, &I->d_hi)) ||
         (e = cudaMemcpyAsync(d_meshoff, mesh_off.data(), 4 * (size_t)M, cudaMemcpyHostToDevice, s)))
         return fail("output", e);
-    k_write<<<(n_rec + 255) / 256, 256, 0, s>>>(d_recs, n_rec, d_meshoff, d_out);
-    std::vector<uint32_t> words(8 * total), stats(4 * (size_t)M);
+    k_write<<<(n_rec + 255) / 256, 256, 0, s>>>(d_recs, n_rec, d_meshoff, I->d_lo, I->d_hi);
+    std::vector<uint32_t> stats(4 * (size_t)M);
     cudaEventRecord(ev1, s);
     if ((e = cudaGetLastError()) ||
-        (e = cudaMemcpyAsync(words.data(), d_out, 32 * total, cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaMemcpyAsync(tri_order.data(), d_order, 4 * N, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaMemcpyAsync(stats.data(), d_stats, 16 * (size_t)M, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
-        return fail("download", e);
+        return fail("output", e);
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ev0, ev1);
     if (device_ms) *device_ms = ms;
     for (uint32_t i = 0; i < M; ++i) {
         GpuTree& t = trees[i];
-        t.nodes.assign(words.begin() + 8 * (size_t)mesh_off[i], words.begin() + 8 * ((size_t)mesh_off[i] + root_recs[i].size));
         t.height = stats[4 * i];
         t.num_inner = stats[4 * i + 1];
         t.num_leaf = stats[4 * i + 2];
@@ -1210,11 +1414,40 @@ int gpu_build_blas(const float* tri_box, uint32_t n_tris, const std::vector<GpuM
     return NOOR_OK;
 }
 
-int gpu_payload_tail(const GpuTailIn& in, GpuTailOut& out, double* device_ms, std::string& err) {
-    auto fail = [&](const char* what, cudaError_t e) {
-        err = std::string("GPU payload: ") + what + ": " + cudaGetErrorString(e);
-        return NOOR_ERR_CUDA;
-    };
+void GpuPayload::download(uint32_t* lo, uint32_t* hi, uint32_t* order) {
+    // the stream of the steps is idle here: trees() ends with a wait for it
+    I->side.join();
+    I->side2.join();
+    if (I->up_error != cudaSuccess) return;  // told by tail()
+    I->side.run([this, lo, hi, order]() {
+        cudaError_t r;
+        (r = cudaSetDevice(I->dev)) ||
+            (r = cudaMemcpyAsync(lo, I->d_lo, 16 * I->n_nodes, cudaMemcpyDeviceToHost, I->s2)) ||
+            (r = cudaMemcpyAsync(order, I->d_order, 4 * (size_t)I->in.n_tris, cudaMemcpyDeviceToHost, I->s2)) ||
+            (r = cudaStreamSynchronize(I->s2));
+        I->down_error = r;
+    });
+    I->side2.run([this, hi]() {
+        cudaError_t r;
+        (r = cudaSetDevice(I->dev)) ||
+            (r = cudaMemcpyAsync(hi, I->d_hi, 16 * I->n_nodes, cudaMemcpyDeviceToHost, I->s3)) ||
+            (r = cudaStreamSynchronize(I->s3));
+        I->down2_error = r;
+    });
+}
+
+int GpuPayload::finish(std::string& err) {
+    I->side.join();
+    I->side2.join();
+    const cudaError_t e = I->down_error != cudaSuccess ? I->down_error : I->down2_error;
+    return e == cudaSuccess ? NOOR_OK : gpu_fail(err, "GPU payload", "download", e);
+}
+
+int GpuPayload::tail(const std::vector<uint32_t>& material_types, double* device_ms, std::string& err) {
+    auto fail = [&](const char* what, cudaError_t e) { return gpu_fail(err, "GPU payload", what, e); };
+    if (I->up_error != cudaSuccess) return fail("upload", I->up_error);
+    const GpuInput& in = I->in;
+    GpuTailOut& out = I->out;
     const size_t T = in.n_tris, C = 3 * T;
     if (C >= 0x7fffffffu) {
         err = "GPU payload: too many triangles";
@@ -1223,48 +1456,30 @@ int gpu_payload_tail(const GpuTailIn& in, GpuTailOut& out, double* device_ms, st
     size_t cap = 16;
     while (cap < 2 * C) cap <<= 1;
     const uint32_t nblk = (uint32_t)((C + kScanBlock - 1) / kScanBlock);
-    cudaStream_t s;
-    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (e != cudaSuccess) return fail("stream", e);
-    struct StreamGuard {
-        cudaStream_t s;
-        ~StreamGuard() { cudaStreamDestroy(s); }
-    } sg{s};
-    keep_pool();
+    cudaStream_t s = I->s;
+    cudaError_t e;
     TimingEvents te;
     if ((e = te.create())) return fail("events", e);
     cudaEvent_t ev0 = te.a, ev1 = te.b;
-    DevBuf b_order, b_vi, b_ni, b_ui, b_vtx, b_nrm, b_uv, b_mi, b_mt, b_slots, b_pmin, b_cs, b_flag, b_first, b_sums,
-        b_total, b_fail, b_ovtx, b_onrm, b_ouv, b_w0, b_w1, b_w2, b_attr;
-    uint32_t *d_order, *d_vi, *d_ni, *d_ui, *d_mi, *d_mt, *d_slots, *d_pmin, *d_cs, *d_flag, *d_first, *d_sums,
-        *d_total, *d_fail;
-    float4 *d_vtx, *d_nrm, *d_ovtx, *d_onrm;
-    float2 *d_uv, *d_ouv;
+    DevBuf b_mt, b_slots, b_pmin, b_cs, b_flag, b_first, b_sums, b_total, b_fail, b_ovtx, b_onrm, b_ouv, b_w0, b_w1,
+        b_w2, b_attr;
+    uint32_t *d_mt, *d_slots, *d_pmin, *d_cs, *d_flag, *d_first, *d_sums, *d_total, *d_fail;
+    float4 *d_ovtx, *d_onrm;
+    float2* d_ouv;
     uint4 *d_w0, *d_w1, *d_w2, *d_attr;
-    if ((e = dalloc(s, b_order, T, &d_order)) || (e = dalloc(s, b_vi, C, &d_vi)) || (e = dalloc(s, b_ni, C, &d_ni)) ||
-        (e = dalloc(s, b_ui, C, &d_ui)) || (e = dalloc(s, b_vtx, in.n_vertices, &d_vtx)) ||
-        (e = dalloc(s, b_nrm, in.n_normals, &d_nrm)) || (e = dalloc(s, b_uv, in.n_uvs, &d_uv)) ||
-        (e = dalloc(s, b_mi, T, &d_mi)) || (e = dalloc(s, b_mt, in.n_materials, &d_mt)) ||
-        (e = dalloc(s, b_slots, cap, &d_slots)) || (e = dalloc(s, b_pmin, cap, &d_pmin)) || (e = dalloc(s, b_cs, C, &d_cs)) ||
+    if ((e = dalloc(s, b_mt, material_types.size(), &d_mt)) || (e = dalloc(s, b_slots, cap, &d_slots)) ||
+        (e = dalloc(s, b_pmin, cap, &d_pmin)) || (e = dalloc(s, b_cs, C, &d_cs)) ||
         (e = dalloc(s, b_flag, C, &d_flag)) || (e = dalloc(s, b_first, C, &d_first)) ||
         (e = dalloc(s, b_sums, nblk, &d_sums)) || (e = dalloc(s, b_total, 1, &d_total)) ||
         (e = dalloc(s, b_fail, 1, &d_fail)) || (e = dalloc(s, b_w0, T, &d_w0)) || (e = dalloc(s, b_w1, T, &d_w1)) ||
         (e = dalloc(s, b_w2, T, &d_w2)) || (e = dalloc(s, b_attr, T, &d_attr)))
         return fail("allocation", e);
     cudaEventRecord(ev0, s);
-    if ((e = cudaMemcpyAsync(d_order, in.tri_order, 4 * T, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_vi, in.vindices, 4 * C, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_ni, in.nindices, 4 * C, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_ui, in.uvindices, 4 * C, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_vtx, in.vertices, 16 * (size_t)in.n_vertices, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_nrm, in.normals, 16 * (size_t)in.n_normals, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_uv, in.uvs, 8 * (size_t)in.n_uvs, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_mi, in.material_indices, 4 * T, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_mt, in.material_types, 4 * (size_t)in.n_materials, cudaMemcpyHostToDevice, s)) ||
+    if ((e = cudaMemcpyAsync(d_mt, material_types.data(), 4 * material_types.size(), cudaMemcpyHostToDevice, s)) ||
         (e = cudaMemsetAsync(d_slots, 0xff, 4 * cap, s)) || (e = cudaMemsetAsync(d_pmin, 0xff, 4 * cap, s)) ||
         (e = cudaMemsetAsync(d_fail, 0, 4, s)))
         return fail("upload", e);
-    TailArgs A{d_order, d_vi, d_ni, d_ui, (uint32_t)C, d_slots, d_pmin, d_cs, (uint32_t)(cap - 1), d_fail};
+    TailArgs A{I->d_order, I->d_vi, I->d_ni, I->d_ui, (uint32_t)C, d_slots, d_pmin, d_cs, (uint32_t)(cap - 1), d_fail};
     const uint32_t g = (uint32_t)((C + 255) / 256);
     k_dedup_insert<<<g, 256, 0, s>>>(A);
     k_dedup_flags<<<g, 256, 0, s>>>(A, d_flag);
@@ -1281,14 +1496,13 @@ int gpu_payload_tail(const GpuTailIn& in, GpuTailOut& out, double* device_ms, st
     }
     if ((e = dalloc(s, b_ovtx, nv, &d_ovtx)) || (e = dalloc(s, b_onrm, nv, &d_onrm)) || (e = dalloc(s, b_ouv, nv, &d_ouv)))
         return fail("allocation", e);
-    k_dedup_vertices<<<g, 256, 0, s>>>(A, d_flag, d_first, d_vtx, d_nrm, d_uv, d_ovtx, d_onrm, d_ouv);
-    k_wald<<<(uint32_t)((T + 255) / 256), 256, 0, s>>>(A, d_first, (uint32_t)T, d_ovtx, d_mi, d_mt, d_w0, d_w1, d_w2,
+    k_dedup_vertices<<<g, 256, 0, s>>>(A, d_flag, d_first, I->d_vtx, I->d_nrm, I->d_uv, d_ovtx, d_onrm, d_ouv);
+    k_wald<<<(uint32_t)((T + 255) / 256), 256, 0, s>>>(A, d_first, (uint32_t)T, d_ovtx, I->d_mi, d_mt, d_w0, d_w1, d_w2,
                                                        d_attr);
     cudaEventRecord(ev1, s);
     out.vertices.resize(4 * (size_t)nv);
     out.normals.resize(4 * (size_t)nv);
     out.uvs.resize(2 * (size_t)nv);
-    for (auto* w : {&out.wald[0], &out.wald[1], &out.wald[2], &out.attr}) w->resize(4 * T);
     if ((e = cudaGetLastError()) ||
         (e = cudaMemcpyAsync(out.vertices.data(), d_ovtx, 16 * (size_t)nv, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaMemcpyAsync(out.normals.data(), d_onrm, 16 * (size_t)nv, cudaMemcpyDeviceToHost, s)) ||

@@ -3,13 +3,16 @@
 // same bytes as the host builder (scene_build.cpp).
 #pragma once
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
+#include "host_array.h"
+
 namespace nbg {
 
-// one source mesh: its slice of the triangle order and the boxes the host
-// computed for it (Model::computeBBoxes)
+// one source mesh: its slice of the triangle order, and the boxes of its
+// triangles and of their centroids (Model::computeBBoxes)
 struct GpuMesh {
     uint32_t start, count;
     float box[6];   // lo xyz, hi xyz
@@ -19,25 +22,12 @@ struct GpuBvhParams {
     uint32_t num_bins, max_height, min_leaf, max_leaf;
     float Ci, Ct;
 };
-// one mesh's tree: 8 words per node in depth-first order, right-child
-// indices relative to the tree's first node
+// one mesh's tree: its first node's index in the scene's node array
 struct GpuTree {
-    std::vector<uint32_t> nodes;
-    uint32_t height = 0, num_inner = 0, num_leaf = 0, max_leaf_tris = 0;
+    uint32_t first = 0, height = 0, num_inner = 0, num_leaf = 0, max_leaf_tris = 0;
 };
-
-// tri_box: 6 floats per triangle (lo, hi); tri_order: the identity on entry,
-// each mesh's slice permuted as the host build leaves it on return
-int gpu_build_blas(const float* tri_box, uint32_t n_tris, const std::vector<GpuMesh>& meshes,
-                   const GpuBvhParams& p, std::vector<uint32_t>& tri_order, std::vector<GpuTree>& trees,
-                   double* device_ms, std::string& err);
-
-// The rest of Model::loadCudaPayload on the device (model.cpp:333-458):
-// vertex de-duplication in BVH order (the first occurrence of a (vertex,
-// normal, uv) index triple gets the next index) and the Wald records and
-// attribute words of each triangle in BVH order.
-struct GpuTailIn {
-    const uint32_t* tri_order;
+// the scene's arrays on the host; they outlive the build
+struct GpuInput {
     uint32_t n_tris;
     const uint32_t *vindices, *nindices, *uvindices;  // 3 per source triangle
     const float* vertices;                            // float4
@@ -47,13 +37,46 @@ struct GpuTailIn {
     const float* uvs;  // float2
     uint32_t n_uvs;
     const uint32_t* material_indices;  // per source triangle
-    const uint32_t* material_types;    // per material
-    uint32_t n_materials;
 };
 struct GpuTailOut {
-    std::vector<float> vertices, normals, uvs;
-    std::vector<uint32_t> wald[3], attr;
+    nbh::HostArray<float> vertices, normals, uvs;
+    nbh::HostArray<uint32_t> wald[3], attr;
 };
-int gpu_payload_tail(const GpuTailIn& in, GpuTailOut& out, double* device_ms, std::string& err);
+
+// One payload's build, its steps in this order.  The scene's arrays go to the
+// device once, the triangle boxes and the triangle order never leave it
+// between the steps, and two more host threads carry what the steps do not
+// wait for: the arrays that only tail() reads go up during boxes() and
+// trees(), while the pages of tail()'s output are taken from the system; the
+// nodes come down during tail().
+class GpuPayload {
+public:
+    // out outlives the build; its wald and attr hold 4 words per triangle
+    GpuPayload(const GpuInput& in, GpuTailOut& out);
+    ~GpuPayload();
+    GpuPayload(const GpuPayload&) = delete;
+    GpuPayload& operator=(const GpuPayload&) = delete;
+    // box and cbox of each mesh from its start and count
+    int boxes(std::vector<GpuMesh>& meshes, std::string& err);
+    // the trees of the meshes, right-child words counted from the scene's
+    // first node; lead[i] nodes of other trees stand before tree i (and after
+    // tree i - 1's), `others` in all
+    int trees(const std::vector<GpuMesh>& meshes, const GpuBvhParams& p, const std::vector<uint32_t>& lead,
+              uint32_t others, std::vector<GpuTree>& trees, double* device_ms, std::string& err);
+    // starts the copy of the nodes (4 words of lo and 4 of hi each, the other trees' places left
+    // undefined) and of the triangle order, done at finish(); after trees()
+    // and before tail()
+    void download(uint32_t* lo, uint32_t* hi, uint32_t* order);
+    // The rest of Model::loadCudaPayload (model.cpp:333-458): vertex
+    // de-duplication in BVH order (the first occurrence of a (vertex, normal,
+    // uv) index triple gets the next index) and the Wald records and attribute
+    // words of each triangle in BVH order.
+    int tail(const std::vector<uint32_t>& material_types, double* device_ms, std::string& err);
+    int finish(std::string& err);
+
+private:
+    struct Impl;
+    std::unique_ptr<Impl> I;
+};
 
 }  // namespace nbg

@@ -36,6 +36,7 @@
 
 #include "../../include/noor_b200.h"
 #include "bvh_gpu.h"
+#include "host_array.h"
 #include "host_common.h"
 
 namespace nbh {
@@ -284,6 +285,30 @@ static void parallel_for(uint32_t n, const F& f) {
     for (auto& th : pool) th.join();
 }
 
+// f(begin, end) over [0, n) in runs of 65536 and more, one per host thread;
+// where no thread can be had the caller does its run itself
+template <class F>
+static void parallel_ranges(size_t n, const F& f) {
+    const size_t nt = std::max<size_t>(1, std::min<size_t>(std::thread::hardware_concurrency(), n / 65536));
+    const size_t chunk = (n + nt - 1) / nt;
+    std::vector<std::thread> pool;
+    try {
+        pool.reserve(nt);
+    } catch (const std::bad_alloc&) {
+        return f(0, n);
+    }
+    for (size_t b = chunk; b < n; b += chunk) {
+        const size_t e = std::min(n, b + chunk);
+        try {
+            pool.emplace_back([&f, b, e]() { f(b, e); });
+        } catch (const std::exception&) {
+            f(b, e);
+        }
+    }
+    f(0, std::min(n, chunk));
+    for (auto& th : pool) th.join();
+}
+
 struct Range {
     uint32_t* b;
     uint32_t* e;
@@ -339,19 +364,29 @@ struct GpuBuildError {
 
 class Builder {
 public:
-    Builder(const noor_scene_desc& d, bool gpu) : D(d), use_gpu(gpu) {}
+    Builder(const noor_scene_desc& d, nbg::GpuPayload* gpu) : D(d), gpu(gpu) {}
 
     const noor_scene_desc& D;
-    bool use_gpu;  // bottom-level trees built on the current CUDA device
+    nbg::GpuPayload* gpu;  // bottom-level trees built on the current CUDA device, or null
     // host trees: subtrees of large ranges above this level are built on
     // threads of their own (when meshes are fewer than threads)
     uint32_t par_levels = 0;
     static constexpr uint32_t kParMinTris = 32768;
     std::vector<Box> tri_box;
     std::vector<MeshInfo> meshes;
+    std::vector<nbg::GpuMesh> gpu_meshes;  // the triangle meshes in order, for the device
     Box scene_box, scene_cbox;
-    std::vector<uint32_t> tri_order, mesh_order, mesh_start;
-    std::vector<uint32_t> nodes;  // the final node array: mesh trees in mesh order, then the top tree
+    HostArray<uint32_t> tri_order;
+    std::vector<uint32_t> mesh_order, mesh_start;
+    // the final node arrays: mesh trees in mesh order, then the top tree
+    HostArray<uint32_t> node_lo, node_hi;
+    // trees built on the host, with their nodes' final place (the device's
+    // nodes are copied around them)
+    struct Placed {
+        uint32_t off;
+        std::vector<uint32_t> nodes;
+    };
+    std::vector<Placed> placed;
     uint32_t root = 0;
     noor_build_stat stat{};
     double gpu_ms = 0.0;
@@ -364,12 +399,31 @@ public:
     // Model::computeBBoxes (model.cpp:73-108); light meshes take the bounds
     // of their shape (CudaShape::getBounds, shape.cuh:71-90)
     void compute_boxes() {
-        tri_box.resize(D.num_triangles);
         meshes.resize(D.num_meshes);
-        for (uint32_t i = 0; i < D.num_meshes; ++i) {
+        if (gpu) {
+            for (uint32_t i = 0; i < D.num_meshes; ++i) {
+                const noor_mesh& m = D.meshes[i];
+                if (m.light_idx >= 0 || m.instance >= 0) continue;
+                nbg::GpuMesh g{m.tri_start, m.tri_count, {}, {}};
+                std::memcpy(g.box, &meshes[i].box, 24);
+                std::memcpy(g.cbox, &meshes[i].cbox, 24);
+                gpu_meshes.push_back(g);
+            }
+            static_assert(sizeof(Box) == 24, "Box is 6 floats");
+            std::string err;
+            if (const int rc = gpu->boxes(gpu_meshes, err)) throw GpuBuildError{rc, err};
+        } else {
+            tri_box.resize(D.num_triangles);
+        }
+        for (uint32_t i = 0, k = 0; i < D.num_meshes; ++i) {
             const noor_mesh& m = D.meshes[i];
             meshes[i].src = &m;
             if (m.light_idx >= 0 || m.instance >= 0) continue;
+            if (gpu) {
+                std::memcpy(&meshes[i].box, gpu_meshes[k].box, 24);
+                std::memcpy(&meshes[i].cbox, gpu_meshes[k++].cbox, 24);
+                continue;
+            }
             Box mb, mc;
             for (uint32_t t = m.tri_start; t < m.tri_start + m.tri_count; ++t) {
                 Box tb;
@@ -529,7 +583,6 @@ public:
         return num_nodes(w) - 1;
     }
     static uint32_t num_nodes(const Work& w) { return w.base + (uint32_t)(w.nodes.size() / 8); }
-    uint32_t num_nodes() const { return (uint32_t)(nodes.size() / 8); }
 
     // BVH::makeLeaf (bvh.cpp:88-153)
     uint32_t make_leaf(Work& w, const Range& r, uint32_t level) {
@@ -625,7 +678,8 @@ public:
     // they are the same bytes as the reference's one-after-another build.
     void build_all() {
         tri_order.resize(D.num_triangles);
-        for (uint32_t i = 0; i < D.num_triangles; ++i) tri_order[i] = i;
+        if (!gpu)
+            for (uint32_t i = 0; i < D.num_triangles; ++i) tri_order[i] = i;
         mesh_order.resize(D.num_meshes);
         for (uint32_t i = 0; i < D.num_meshes; ++i) mesh_order[i] = i;
         mesh_start.assign(D.num_meshes, 0u);
@@ -637,43 +691,8 @@ public:
             if (D.meshes[i].instance < 0) src.push_back(i);
         std::vector<Work> trees(src.size());
         std::vector<char> done(src.size(), 0);
-        if (use_gpu) {
-            // the triangle meshes on the device (bvh_gpu.cu), the light
-            // meshes' one-leaf trees below
-            std::vector<nbg::GpuMesh> gm;
-            std::vector<size_t> gj;
-            for (size_t j = 0; j < src.size(); ++j) {
-                const noor_mesh& m = D.meshes[src[j]];
-                if (m.light_idx >= 0) continue;
-                nbg::GpuMesh g;
-                g.start = m.tri_start;
-                g.count = m.tri_count;
-                const MeshInfo& mi = meshes[src[j]];
-                const float b[12] = {mi.box.lo.x,  mi.box.lo.y,  mi.box.lo.z,  mi.box.hi.x,  mi.box.hi.y,  mi.box.hi.z,
-                                     mi.cbox.lo.x, mi.cbox.lo.y, mi.cbox.lo.z, mi.cbox.hi.x, mi.cbox.hi.y, mi.cbox.hi.z};
-                std::memcpy(g.box, b, 24);
-                std::memcpy(g.cbox, b + 6, 24);
-                gm.push_back(g);
-                gj.push_back(j);
-            }
-            nbg::GpuBvhParams bp{D.bvh.num_bins, D.bvh.max_height, D.bvh.min_leaf_tris, D.bvh.max_leaf_tris,
-                                 D.bvh.Ci, D.bvh.Ct};
-            std::vector<nbg::GpuTree> gt;
-            std::string err;
-            static_assert(sizeof(Box) == 24, "Box is 6 floats");
-            const int rc = nbg::gpu_build_blas(reinterpret_cast<const float*>(tri_box.data()), D.num_triangles, gm, bp,
-                                               tri_order, gt, &gpu_ms, err);
-            if (rc) throw GpuBuildError{rc, err};
-            for (size_t k = 0; k < gj.size(); ++k) {
-                Work& w = trees[gj[k]];
-                w.nodes = std::move(gt[k].nodes);
-                w.stat.height = gt[k].height;
-                w.stat.num_inner_nodes = gt[k].num_inner;
-                w.stat.num_leaf_nodes = gt[k].num_leaf;
-                w.stat.max_leaf_tris = gt[k].max_leaf_tris;
-                done[gj[k]] = 1;
-            }
-        }
+        if (gpu)  // the triangle meshes on the device (bvh_gpu.cu), the light meshes' one-leaf trees here
+            for (size_t j = 0; j < src.size(); ++j) done[j] = D.meshes[src[j]].light_idx < 0;
         {
             size_t todo = 0;
             for (size_t j = 0; j < src.size(); ++j) todo += done[j] ? 0 : 1;
@@ -707,34 +726,80 @@ public:
         for (auto& t : pool) t.join();
         for (auto& e : errs)
             if (e) std::rethrow_exception(e);
-        size_t total = 0;
-        for (const Work& w : trees) total += w.nodes.size();
-        nodes.reserve(total + 8 * (size_t)2 * (D.num_meshes + 1));
-        for (size_t j = 0; j < src.size(); ++j) {
+        std::vector<nbg::GpuTree> gt;
+        if (gpu) {
+            std::vector<uint32_t> lead;
+            uint32_t others = 0, since = 0;
+            for (size_t j = 0; j < src.size(); ++j) {
+                if (done[j]) {
+                    lead.push_back(since);
+                    since = 0;
+                } else {
+                    since += num_nodes(trees[j]);
+                    others += num_nodes(trees[j]);
+                }
+            }
+            const nbg::GpuBvhParams bp{D.bvh.num_bins, D.bvh.max_height, D.bvh.min_leaf_tris, D.bvh.max_leaf_tris,
+                                       D.bvh.Ci, D.bvh.Ct};
+            std::string err;
+            if (const int rc = gpu->trees(gpu_meshes, bp, lead, others, gt, &gpu_ms, err)) throw GpuBuildError{rc, err};
+        }
+        uint32_t total = 0;
+        for (size_t j = 0, k = 0; j < src.size(); ++j) {
             Work& w = trees[j];
-            const uint32_t off = num_nodes();
-            mesh_start[src[j]] = off;
-            for (size_t n = 0; n < w.nodes.size(); n += 8)
-                if (!(w.nodes[n + 7] & NOOR_TRI_LEAF_MASK)) w.nodes[n + 3] += off;  // inner: right child
-            nodes.insert(nodes.end(), w.nodes.begin(), w.nodes.end());
+            if (done[j]) {
+                const nbg::GpuTree& g = gt[k++];
+                w.stat.height = g.height;
+                w.stat.num_inner_nodes = g.num_inner;
+                w.stat.num_leaf_nodes = g.num_leaf;
+                w.stat.max_leaf_tris = g.max_leaf_tris;
+                total = g.first + g.num_inner + g.num_leaf;
+                mesh_start[src[j]] = g.first;
+            } else {
+                mesh_start[src[j]] = total;
+                for (size_t n = 0; n < w.nodes.size(); n += 8)
+                    if (!(w.nodes[n + 7] & NOOR_TRI_LEAF_MASK)) w.nodes[n + 3] += total;  // inner: right child
+                placed.push_back(Placed{total, std::move(w.nodes)});
+                total += (uint32_t)(placed.back().nodes.size() / 8);
+            }
             stat.height = std::max(stat.height, w.stat.height);
             stat.num_inner_nodes += w.stat.num_inner_nodes;
             stat.num_leaf_nodes += w.stat.num_leaf_nodes;
             stat.max_leaf_tris = std::max(stat.max_leaf_tris, w.stat.max_leaf_tris);
-            std::vector<uint32_t>().swap(w.nodes);
         }
         for (uint32_t i = 0; i < D.num_meshes; ++i)
             if (D.meshes[i].instance >= 0) mesh_start[i] = mesh_start[D.meshes[i].instance];
-        root = num_nodes();
+        root = total;
         Work top;
         top.init(D.bvh.num_bins);
         top.base = root;
         top.stat = stat;
         Range r{mesh_order.data(), mesh_order.data() + D.num_meshes, scene_box, scene_cbox, kMeshBin};
         build(top, r, stat.height);
-        nodes.insert(nodes.end(), top.nodes.begin(), top.nodes.end());
         stat = top.stat;
         stat.height += 1;
+        total += (uint32_t)(top.nodes.size() / 8);
+        placed.push_back(Placed{root, std::move(top.nodes)});
+        node_lo.resize(4 * (size_t)total);
+        node_hi.resize(4 * (size_t)total);
+        if (gpu)
+            gpu->download(node_lo.data(), node_hi.data(), tri_order.data());
+        else
+            place_nodes();
+    }
+
+    // the host's trees into the node arrays (once the device's nodes, whose
+    // copy covers these places too, have come)
+    void place_nodes() {
+        for (Placed& t : placed) {
+            uint32_t* lo = node_lo.data() + 4 * (size_t)t.off;
+            uint32_t* hi = node_hi.data() + 4 * (size_t)t.off;
+            for (size_t n = 0; n < t.nodes.size(); n += 8) {
+                std::memcpy(lo + n / 2, t.nodes.data() + n, 16);
+                std::memcpy(hi + n / 2, t.nodes.data() + n + 4, 16);
+            }
+            std::vector<uint32_t>().swap(t.nodes);
+        }
     }
 };
 
@@ -781,11 +846,11 @@ static void wald_record(const V3& A, const V3& B, const V3& C, uint32_t* r0, uin
 using namespace nbh;
 
 struct noor_payload_handle {
-    std::vector<uint32_t> attr;
-    std::vector<float> vertices, normals, uvs;
+    nbh::HostArray<uint32_t> attr;
+    nbh::HostArray<float> vertices, normals, uvs;
     std::vector<float> xf[9];
-    std::vector<uint32_t> wald[3];
-    std::vector<uint32_t> bvh_lo, bvh_hi;
+    nbh::HostArray<uint32_t> wald[3];
+    nbh::HostArray<uint32_t> bvh_lo, bvh_hi;
     uint32_t root = 0;
     std::vector<std::vector<float>> tex_data;
     std::vector<noor_texture> tex_meta;       // width, height, filter, address of each texture
@@ -795,7 +860,7 @@ struct noor_payload_handle {
     std::vector<noor_spot_light> spot_lights;
     std::vector<noor_distant_light> distant_lights;
     std::vector<noor_material> materials;
-    std::vector<uint32_t> tri_order;
+    nbh::HostArray<uint32_t> tri_order;
     uint32_t num_tris = 0;
     uint32_t height = 0;
     float scene_radius = 0.0f;
@@ -813,6 +878,31 @@ static uint32_t add_image(noor_payload_handle* h, const noor_image& im, int32_t 
     h->tex_data.emplace_back(im.rgba, im.rgba + 4 * (size_t)im.width * im.height);
     h->tex_meta.push_back(noor_texture{im.width, im.height, nullptr, filter, NOOR_ADDRESS_WRAP});
     return (uint32_t)h->tex_data.size() - 1;
+}
+
+// Indices and vertices of a scene, checked on all host threads (1.3M
+// triangles: one thread took 10 ms).  The loops have no early way out, so they
+// run at the speed of memory.
+enum : uint32_t { kBadIndex = 1u, kBadVertex = 2u, kBadMaterial = 4u };
+static uint32_t check_arrays(const noor_scene_desc* d) {
+    std::atomic<uint32_t> bad{0u};
+    parallel_ranges(d->num_triangles, [&](size_t b, size_t e) {
+        uint32_t v = 0, n = 0, u = 0, m = 0;
+        for (size_t i = 3 * b; i < 3 * e; ++i) {
+            v = std::max(v, d->vindices[i]);
+            n = std::max(n, d->nindices[i]);
+            u = std::max(u, d->uvindices[i]);
+        }
+        for (size_t i = b; i < e; ++i) m = std::max(m, d->material_indices[i]);
+        if (v >= d->num_vertices || n >= d->num_normals || u >= d->num_uvs) bad |= kBadIndex;
+        if (m >= d->num_materials) bad |= kBadMaterial;
+    });
+    parallel_ranges(d->num_vertices, [&](size_t b, size_t e) {
+        bool finite = true;  // exponent bits not all ones
+        for (size_t i = 4 * b; i < 4 * e; ++i) finite &= (f2u(d->vertices[i]) & 0x7f800000u) != 0x7f800000u;
+        if (!finite) bad |= kBadVertex;
+    });
+    return bad;
 }
 
 static int build_payload(const noor_scene_desc* d, bool gpu, noor_payload_handle** out, noor_build_stat* stat) {
@@ -848,15 +938,10 @@ static int build_payload(const noor_scene_desc* d, bool gpu, noor_payload_handle
         next += m.tri_count;
     }
     if (next != d->num_triangles) return set_error(NOOR_ERR_INVALID, "noor_build_payload: meshes do not cover triangles");
-    for (size_t i = 0; i < 3 * (size_t)d->num_triangles; ++i) {
-        if (d->vindices[i] >= d->num_vertices || d->nindices[i] >= d->num_normals || d->uvindices[i] >= d->num_uvs)
-            return set_error(NOOR_ERR_INVALID, "noor_build_payload: vertex attribute index out of range");
-    }
-    for (size_t i = 0; i < 4 * (size_t)d->num_vertices; ++i)
-        if (!std::isfinite(d->vertices[i])) return set_error(NOOR_ERR_INVALID, "noor_build_payload: non-finite vertex");
-    for (uint32_t i = 0; i < d->num_triangles; ++i)
-        if (d->material_indices[i] >= d->num_materials)
-            return set_error(NOOR_ERR_INVALID, "noor_build_payload: material index out of range");
+    const uint32_t bad = check_arrays(d);
+    if (bad & kBadIndex) return set_error(NOOR_ERR_INVALID, "noor_build_payload: vertex attribute index out of range");
+    if (bad & kBadVertex) return set_error(NOOR_ERR_INVALID, "noor_build_payload: non-finite vertex");
+    if (bad & kBadMaterial) return set_error(NOOR_ERR_INVALID, "noor_build_payload: material index out of range");
     if (d->num_images && !d->images) return set_error(NOOR_ERR_INVALID, "noor_build_payload: image count without an array");
     for (uint32_t i = 0; i < d->num_images; ++i)
         if (d->images[i].width <= 0 || d->images[i].height <= 0 || !d->images[i].rgba)
@@ -870,7 +955,18 @@ static int build_payload(const noor_scene_desc* d, bool gpu, noor_payload_handle
     std::unique_ptr<noor_payload_handle> h(new (std::nothrow) noor_payload_handle());
     if (!h) return set_error(NOOR_ERR_OOM, "noor_build_payload: out of host memory");
     try {
-        Builder B(*d, gpu);
+        nbg::GpuTailOut tail_out;
+        Builder B(*d, nullptr);
+        std::unique_ptr<nbg::GpuPayload> G;  // its side threads write into the two above: gone before them
+        if (gpu) {
+            for (auto* w : {&tail_out.wald[0], &tail_out.wald[1], &tail_out.wald[2], &tail_out.attr})
+                w->resize(4 * (size_t)d->num_triangles);
+            G.reset(new nbg::GpuPayload(nbg::GpuInput{d->num_triangles, d->vindices, d->nindices, d->uvindices,
+                                                      d->vertices, d->num_vertices, d->normals, d->num_normals, d->uvs,
+                                                      d->num_uvs, d->material_indices},
+                                        tail_out));
+            B.gpu = G.get();
+        }
         B.compute_boxes();
         const auto t1 = std::chrono::steady_clock::now();
         B.build_all();
@@ -879,17 +975,8 @@ static int build_payload(const noor_scene_desc* d, bool gpu, noor_payload_handle
         h->num_tris = d->num_triangles;
         h->root = B.root;
         h->height = B.stat.height;
-        h->tri_order = B.tri_order;
         h->scene_radius = B.scene_box.radius();
         h->skydome_type = d->skydome_type;
-        const uint32_t nn = B.num_nodes();
-        h->bvh_lo.resize(4 * (size_t)nn);
-        h->bvh_hi.resize(4 * (size_t)nn);
-        for (uint32_t i = 0; i < nn; ++i)
-            for (int k = 0; k < 4; ++k) {
-                h->bvh_lo[4 * (size_t)i + k] = B.nodes[8 * (size_t)i + k];
-                h->bvh_hi[4 * (size_t)i + k] = B.nodes[8 * (size_t)i + 4 + k];
-            }
         // transforms in mesh_order (BVH::loadCudaPayload, bvh.cpp:59-85)
         for (int k = 0; k < 9; ++k) h->xf[k].reserve(4 * (size_t)d->num_meshes);
         for (uint32_t i = 0; i < d->num_meshes; ++i) {
@@ -1017,13 +1104,12 @@ static int build_payload(const noor_scene_desc* d, bool gpu, noor_payload_handle
             // the same steps on the device (bvh_gpu.cu)
             std::vector<uint32_t> mtypes(d->num_materials);
             for (uint32_t i = 0; i < d->num_materials; ++i) mtypes[i] = h->materials[i].type;
-            nbg::GpuTailIn ti{B.tri_order.data(), d->num_triangles, d->vindices, d->nindices, d->uvindices,
-                              d->vertices, d->num_vertices, d->normals, d->num_normals, d->uvs, d->num_uvs,
-                              d->material_indices, mtypes.data(), d->num_materials};
-            nbg::GpuTailOut to;
+            nbg::GpuTailOut& to = tail_out;
             std::string err;
-            const int rc = nbg::gpu_payload_tail(ti, to, &tail_ms, err);
+            int rc = G->tail(mtypes, &tail_ms, err);
+            if (rc == NOOR_OK) rc = G->finish(err);
             if (rc) return set_error(rc, err);
+            B.place_nodes();
             h->vertices = std::move(to.vertices);
             h->normals = std::move(to.normals);
             h->uvs = std::move(to.uvs);
@@ -1073,6 +1159,9 @@ static int build_payload(const noor_scene_desc* d, bool gpu, noor_payload_handle
                 a[3] = mi;
             });
         }
+        h->tri_order = std::move(B.tri_order);
+        h->bvh_lo = std::move(B.node_lo);
+        h->bvh_hi = std::move(B.node_hi);
         const auto t4 = std::chrono::steady_clock::now();
         if (stat) {
             *stat = B.stat;

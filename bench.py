@@ -384,7 +384,7 @@ def reference_hosek(capi, h):
 
 
 class MegakernelPath:
-    """reference-facing path: noor_render_frames (the megakernel) into the
+    """reference-facing path: noor_render_frames (the megakernel's paths) into the
     context film; e2e adds update_cuda_camera and noor_get_framebuffer"""
 
     name = "megakernel"

@@ -396,7 +396,7 @@ int noor_tonemap_device(const float* d_film_rgba, size_t n_pixels, int op, float
  * reference's GL window), any other op writes a binary PPM of the tonemapped
  * film, top row first. */
 int noor_save_image(const char* path, int op, float exposure);
-/* Rays traced by the megakernel since the last reset (device counters):
+/* Rays traced by the renders since the last reset (device counters):
  * [0] extension (closest-hit) rays, [1] shadow (any-hit) rays, [2] paths. */
 int noor_ray_counters(uint64_t counters[3], int reset);
 /* Device status word (NOOR_DEV_* bits) accumulated since the last reset. */
@@ -597,7 +597,7 @@ typedef struct noor_build_stat {
     float scene_max[3];
     float scene_radius;
     double build_seconds;        /* the whole call                           */
-    double box_seconds;          /* triangle and mesh boxes (host)           */
+    double box_seconds;          /* boxes: host, or GPU with their uploads   */
     double tree_seconds;         /* the trees: host, or GPU with transfers   */
     double tree_device_ms;       /* GPU build: device time of the trees      */
     double tail_seconds;         /* vertex de-duplication, Wald records      */

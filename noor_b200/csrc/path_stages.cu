@@ -25,7 +25,19 @@ NB_D void stage_kahan(float3& sum, float3& c, const float3& x) {
 // running mean.  The chunk in progress at the end of a batch is kept in
 // part_sum / part_comp.
 __global__ void __launch_bounds__(256) st_fold(DevCamera C, StageDev W, StageFold F) {
+    stage_follow();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q == 0) {
+        // ray counts of the batch (extend traced every active path of a bounce)
+        unsigned long long ext = W.paths, sh = 0;
+        for (uint32_t b = 0; b < F.bounces; ++b) {
+            if (b) ext += W.count[b * kStWords + kStActive];
+            sh += W.count[b * kStWords + kStShadow];
+        }
+        W.counters[0] += ext;
+        W.counters[1] += sh;
+        W.counters[2] += W.paths;
+    }
     if (q >= C.w * C.h) return;
     const uint32_t pix = stage_pixel(q, C.w, C.h);
     const uint32_t per = (F.total + F.chunks - 1) / F.chunks;
@@ -91,21 +103,17 @@ __global__ void __launch_bounds__(256) st_fold(DevCamera C, StageDev W, StageFol
     }
 }
 
-// ray counts of a batch (extend traced every active path of a bounce)
-__global__ void st_count(StageDev W, uint32_t bounces) {
-    unsigned long long ext = bounces ? W.paths : 0u, sh = 0;
-    for (uint32_t b = 0; b < bounces; ++b) {
-        if (b) ext += W.count[b * kStWords + kStActive];
-        sh += W.count[b * kStWords + kStShadow];
-    }
-    W.counters[0] += ext;
-    W.counters[1] += sh;
-    W.counters[2] += W.paths;
-}
-
 // paths a batch holds at most: 228 bytes of state each (64 more with bump
 // maps), a gigabyte in all; a frame beyond it is left to the megakernel
 constexpr uint32_t kStageMaxPaths = 1u << 22;
+// Scenes with bump maps: fewer paths than this go to the megakernel.  The
+// stages store and load 64 bytes of differentials a bounce and run the largest
+// shading kernel, and below one path a lane the megakernel's latency is the
+// shorter one (one sample of the textured room, megakernel / staged:
+// 128x96 238 / 260 us, 160x120 255 / 274, 192x144 330 / 298); scenes without
+// are at least as fast staged from the smallest frames on (97x61 room 181 /
+// 161 us, sky 166 / 127).
+constexpr uint64_t kStageMinBumpPaths = 20000;
 
 // the batch's buffers, laid out in one allocation that the context keeps.
 // False (nothing changed) where the device has no room for it.
@@ -161,6 +169,7 @@ int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done) 
     *done = false;
     const uint64_t npix = (uint64_t)C.cam.w * C.cam.h;
     if (npix > kStageMaxPaths || S.bounces == 0 || S.bounces > 1024) return NOOR_OK;
+    if (S.has_bump && npix * a.nframes < kStageMinBumpPaths) return NOOR_OK;
     const uint32_t nb = (uint32_t)std::min<uint64_t>(a.nframes, kStageMaxPaths / npix);
     StageDev W{};
     if (!stage_buffers(C, (uint32_t)npix * nb, nb, S.bounces, S.has_bump != 0u, W)) return NOOR_OK;
@@ -171,11 +180,10 @@ int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done) 
         W.paths = (uint32_t)npix * W.frames;
         W.frame0 = a.frame0 + f;
         // the counters and the first hits lie side by side
-        const size_t zero = (char*)(W.first + W.frames) - (char*)W.count;
-        cudaError_t e = cudaMemsetAsync(W.count, 0, zero, C.stream);
-        if (e == cudaSuccess)
-            e = S.isect == NOOR_ISECT_WATERTIGHT ? launch_stages_wt(S, C.cam, W, C.sm_count, &C.launches, C.stream)
-                                                 : launch_stages_wald(S, C.cam, W, C.sm_count, &C.launches, C.stream);
+        W.zero = (uint32_t)(((char*)(W.first + W.frames) - (char*)W.count) / 4);
+        cudaError_t e = S.isect == NOOR_ISECT_WATERTIGHT
+                            ? launch_stages_wt(S, C.cam, W, C.sm_count, &C.launches, C.stream)
+                            : launch_stages_wald(S, C.cam, W, C.sm_count, &C.launches, C.stream);
         if (e != cudaSuccess) return cuda_fail(e, "staged render");
         StageFold F{};
         F.first = f;
@@ -189,11 +197,10 @@ int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done) 
         F.part_sum = a.part_sum;
         F.part_comp = a.part_comp;
         F.lookat = a.lookat;
-        st_fold<<<(uint32_t)((npix + 255) / 256), 256, 0, C.stream>>>(C.cam, W, F);
-        st_count<<<1, 1, 0, C.stream>>>(W, S.bounces);
-        e = cudaGetLastError();
+        F.bounces = S.bounces;
+        e = launch_stage(st_fold, dim3((uint32_t)((npix + 255) / 256)), 256, 0, C.stream, C.cam, W, F);
         if (e != cudaSuccess) return cuda_fail(e, "staged render");
-        C.launches += 2;
+        C.launches += 1;
     }
     *done = true;
     return NOOR_OK;

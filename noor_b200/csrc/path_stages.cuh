@@ -69,6 +69,7 @@ struct StageDev {
     uint32_t paths;     // paths of the batch
     uint32_t frames;    // frames of the batch
     uint32_t frame0;    // number of its first frame
+    uint32_t zero;      // words from count to the end of first
     uint32_t keep;      // paths between the pend and pbeta entries of one bounce and the next (0: reused)
 };
 
@@ -78,6 +79,7 @@ struct StageFold {
     uint32_t chunks;
     uint32_t frame0;    // number of the call's first frame
     uint32_t fresh;
+    uint32_t bounces;
     int film_mode;
     float4* film_sum;
     float4* film_comp;
@@ -133,10 +135,38 @@ NB_D RayDiff stage_load_diff(const StageDev& W, uint32_t i) {
     return r;
 }
 
+// The stages are launched so that a kernel's blocks come to the SMs while the
+// last blocks of the one before still run (programmatic stream serialization),
+// and wait here until it has finished and its writes can be read.
+NB_D void stage_follow() {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+}
+
+// kernel<<<g, b, sm, s>>>(args...), its blocks launched ahead of the end of
+// the kernel before (stage_follow)
+template <class... P, class... A>
+cudaError_t launch_stage(void (*kernel)(P...), dim3 g, uint32_t b, size_t sm, cudaStream_t s, const A&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = g;
+    c.blockDim = dim3(b);
+    c.dynamicSmemBytes = sm;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // path i: pixel slot i / frames, frame i % frames (all samples of a pixel side by side)
 template <bool EXT, bool DIFF>
 __global__ void __launch_bounds__(256) st_begin(DevCamera C, StageDev W) {
+    stage_follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the batch's counters and first hits, which the stages after this one use
+    for (uint32_t z = i; z < W.zero; z += gridDim.x * blockDim.x) W.count[z] = 0u;
     if (i >= W.paths) return;
     const uint32_t pix = stage_pixel(i / W.frames, C.w, C.h);
     Rng rng{tea16(pix, W.frame0 + i % W.frames)};
@@ -155,17 +185,25 @@ __global__ void __launch_bounds__(256) st_begin(DevCamera C, StageDev W) {
     W.hit2[i] = make_uint2(0u, kStDone);
 }
 
+// The next rays of a list of n for this warp.  The first rays of each of the
+// launch's warps are its own by number, so that a short list takes no atomics
+// and an empty one costs a warp one read; the rest are taken as warps get free.
+NB_D uint32_t stage_take(uint32_t* taken, uint32_t warps, uint32_t take, uint32_t n, uint32_t lane) {
+    if (warps * take >= n) return n;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(taken, take);
+    return warps * take + __shfl_sync(0xFFFFFFFFu, base, 0);
+}
+
 template <int ISECT, bool EXT>
 NB_D void stage_extend(const DevScene& S, const DevCamera& C, const StageDev& W, uint32_t bounce, const SmemStack& stk) {
     uint32_t* cnt = W.count + bounce * kStWords;
     const uint32_t n = bounce ? cnt[kStActive] : W.paths;
     const uint32_t* queue = W.queue[bounce & 1u];
     const uint32_t lane = threadIdx.x & 31, take = rays_per_warp(n);
-    for (;;) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(cnt + kStTake, take);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= n) break;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (uint32_t base = warp * take; base < n; base = stage_take(cnt + kStTake, warps, take, n, lane)) {
         if (lane >= take || base + lane >= n) continue;
         const uint32_t i = bounce ? queue[base + lane] : base + lane;
         float tmax = kInf;
@@ -209,18 +247,25 @@ NB_D void stage_pending(const StageDev& W, uint32_t i, float3& L) {
     L += f3(b) * Ld;
 }
 
-// One row of blocks per material kind (blockIdx.y), so that a short queue
-// shades beside a long one
+// The queues of the material kinds one after the other, each filled up to
+// whole warps, dealt to one wave of blocks: every warp shades one kind, a short
+// queue shades beside a long one, and a bounce with nothing to shade costs one
+// read a warp (three rows of 8 blocks per SM, a row per kind: 5.8 us for the
+// empty bounces of a 768x512 frame, against 4.2 for st_trace's one wave).
 // Bound by latency and by instruction fetch at these sizes: 4, 6 or 8 blocks
 // per SM (16 to 32 warps) measure the same (1.10, 1.07, 1.09 ms for four
 // 641x359 frames of the textured room); 6 leaves 80 registers.
 template <int ISECT, bool EXT, bool DIFF>
 __global__ void __launch_bounds__(128, EXT ? 4 : 6) st_shade(DevScene S, StageDev W, uint32_t bounce) {
-    const uint32_t kind_q = blockIdx.y;
+    stage_follow();
     uint32_t* cnt = W.count + bounce * kStWords;
-    const uint32_t n = cnt[kind_q];
+    const uint32_t n0 = cnt[0], n1 = cnt[1], n2 = cnt[2];
+    const uint32_t b1 = (n0 + 31u) & ~31u, b2 = b1 + ((n1 + 31u) & ~31u);
     uint32_t* next = W.queue[(bounce & 1u) ^ 1u];
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < b2 + n2; j += gridDim.x * blockDim.x) {
+        const uint32_t kind_q = j < b1 ? 0u : j < b2 ? 1u : 2u;
+        const uint32_t k = j - (kind_q == 0u ? 0u : kind_q == 1u ? b1 : b2);
+        if (k >= (kind_q == 0u ? n0 : kind_q == 1u ? n1 : n2)) continue;
         const uint32_t i = W.qshade[kind_q * W.cap + k];
         const float4 ow = W.o[i], dw = W.d[i], bw = W.beta[i], Lw = W.L[i], hw = W.hit[i];
         const uint2 h2 = W.hit2[i];
@@ -304,11 +349,9 @@ NB_D void stage_occlude(const DevScene& S, const StageDev& W, uint32_t bounce, c
     uint32_t* cnt = W.count + bounce * kStWords;
     const uint32_t n = cnt[kStShadow];
     const uint32_t lane = threadIdx.x & 31, take = rays_per_warp(n);
-    for (;;) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(cnt + kStTakeShadow, take);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= n) break;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t warp = warps - 1u - (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+    for (uint32_t base = warp * take; base < n; base = stage_take(cnt + kStTakeShadow, warps, take, n, lane)) {
         const uint32_t q = base + lane;
         if (lane >= take || q >= n) continue;
         const StoredRay ray{W.sh_o + q, W.sh_d + q};
@@ -318,24 +361,27 @@ NB_D void stage_occlude(const DevScene& S, const StageDev& W, uint32_t bounce, c
     }
 }
 
-// The rays of a shade step: the next bounce's extension (blockIdx.y 0) beside
-// the shadow rays (blockIdx.y 1), which only the next shade step waits for.
+// The rays of a shade step: the next bounce's extension and the shadow rays,
+// which only the next shade step waits for.  Every warp serves both lists, the
+// extension first, and the lists are dealt out from the two ends of the grid,
+// so that short lists meet on no warp.  One wave of blocks (kStageTraceBlocks
+// per SM): a second one, or a row of blocks per list, only waits to find its
+// list empty in the last bounces.
 // bounce: the shade step's; extend only before the first (bounce -1) and
 // shadow only after the last.
 template <int ISECT, bool EXT>
 __global__ void __launch_bounds__(128, 7) st_trace(DevScene S, DevCamera C, StageDev W, int bounce) {
     extern __shared__ uint32_t smem[];
+    stage_follow();
     const SmemStack stk{smem + threadIdx.x, (int)blockDim.x, S.stack_cap};
-    if (blockIdx.y == 0) {
-        if (bounce + 1 < (int)S.bounces) stage_extend<ISECT, EXT>(S, C, W, (uint32_t)(bounce + 1), stk);
-    } else {
-        stage_occlude<ISECT, EXT>(S, W, (uint32_t)bounce, stk);
-    }
+    if (bounce + 1 < (int)S.bounces) stage_extend<ISECT, EXT>(S, C, W, (uint32_t)(bounce + 1), stk);
+    if (bounce >= 0) stage_occlude<ISECT, EXT>(S, W, (uint32_t)bounce, stk);
 }
 
 // what a path's radiance still lacks; the clamped radiance into L
 template <int ISECT, bool EXT>
 __global__ void __launch_bounds__(256) st_finish(DevScene S, StageDev W) {
+    stage_follow();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= W.paths) return;
     const float4 Lw = W.L[i], bw = W.beta[i];

@@ -6,25 +6,32 @@
 
 namespace nb {
 
+constexpr int kStageTrav = 64, kStageTraceBlocks = 14;  // st_trace: 7 blocks of 128 threads in registers
+
 template <int ISECT, bool EXT, bool DIFF>
 cudaError_t run_stages(const DevScene& S, const DevCamera& C, const StageDev& W, int sm_count, uint64_t* launches,
                        cudaStream_t s) {
-    constexpr int trav = 64;
-    const size_t sm = (size_t)S.stack_words * trav * sizeof(uint32_t);
+    const size_t sm = (size_t)S.stack_words * kStageTrav * sizeof(uint32_t);
     cudaError_t e = cudaFuncSetAttribute(st_trace<ISECT, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     const uint32_t all = (W.paths + 255) / 256;
-    const uint32_t gt = std::min<uint32_t>((W.paths + trav - 1) / trav, (uint32_t)sm_count * 16);
-    const dim3 gs(std::min<uint32_t>((W.paths + 127) / 128, (uint32_t)sm_count * 8), kStageKinds);
-    st_begin<EXT, DIFF><<<all, 256, 0, s>>>(C, W);
-    st_trace<ISECT, EXT><<<gt, trav, sm, s>>>(S, C, W, -1);
-    for (uint32_t b = 0; b < S.bounces; ++b) {
-        st_shade<ISECT, EXT, DIFF><<<gs, 128, 0, s>>>(S, W, b);
-        st_trace<ISECT, EXT><<<dim3(gt, 2), trav, sm, s>>>(S, C, W, (int)b);
-    }
+    // Two paths a warp until there are paths enough, where a walk is all that a
+    // ray does; 32 a warp where lights of every shape and alpha maps come into
+    // it, whose code then runs on fewer SMs (one sample of a 128x96 frame, 2 /
+    // 4 / 16 / 32 a warp: room 178 / 179 / 189 / 209 us, textured room 324 /
+    // 324 / 261 / 270; 192x144: 202 to 216, and 373 / 377 / 360 / 294)
+    constexpr uint32_t kPer = EXT ? 64 : 4;
+    const uint32_t gt = std::min<uint32_t>((W.paths + kPer - 1) / kPer, (uint32_t)(sm_count * kStageTraceBlocks));
+    const uint32_t gs = std::min<uint32_t>((W.paths + 127) / 128, (uint32_t)sm_count * (EXT ? 4 : 6));
+    if ((e = launch_stage(st_begin<EXT, DIFF>, all, 256, 0, s, C, W)) ||
+        (e = launch_stage(st_trace<ISECT, EXT>, gt, kStageTrav, sm, s, S, C, W, -1)))
+        return e;
+    for (uint32_t b = 0; b < S.bounces; ++b)
+        if ((e = launch_stage(st_shade<ISECT, EXT, DIFF>, gs, 128, 0, s, S, W, b)) ||
+            (e = launch_stage(st_trace<ISECT, EXT>, gt, kStageTrav, sm, s, S, C, W, (int)b)))
+            return e;
     *launches += 3 + 2 * (uint64_t)S.bounces;
-    st_finish<ISECT, EXT><<<all, 256, 0, s>>>(S, W);
-    return cudaGetLastError();
+    return launch_stage(st_finish<ISECT, EXT>, all, 256, 0, s, S, W);
 }
 
 template <int ISECT>

@@ -982,14 +982,18 @@ NB_D bool trace_shadow(const DevScene& S, const World& world, float tmax, const 
     return trace_any<ISECT, EXT>(S, o, d, tmax, st, status);
 }
 
-// Rays a warp of this launch takes at a time from a list of n: 32, or fewer
-// where there are more warps than that makes work for -- the lanes of a warp
-// walk one after the other where their walks part, so a short list is spread
-// over the warps (150 us of extension for a few hundred scattered rays 32 to
-// a warp, the last bounces of a 1920x1080 frame, take 20 one to a warp)
+// Rays a warp of this launch takes at a time from a list of n: 32, or up to 4
+// where the launch has warps enough for that -- the lanes of a warp walk one
+// after the other where their walks part, so a short list is spread over the
+// warps (150 us of extension for a few hundred scattered rays 32 to a warp, the
+// last bounces of a 1920x1080 frame, take 20 one to a warp).  Beyond 4 half
+// filled warps cost more issue slots than they save latency (one sample of a
+// 256x256 room, 16 rays a warp: 245 us, 32: 222; of a 768x512 sky scene, 8
+// spheres: 290 and 275)
 NB_D uint32_t rays_per_warp(uint32_t n) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    return min(32u, max(1u, (n + warps - 1u) / warps));
+    const uint32_t take = max(1u, (n + warps - 1u) / warps);
+    return take > 4u ? 32u : take;
 }
 
 // The walks of the adjoint: the four-wide tree where the

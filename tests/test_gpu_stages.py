@@ -51,6 +51,8 @@ CASES = {
     "roughglass": (lambda: _boxes("roughglass", 65, 33), 3),
     "shadowcatcher": (lambda: _boxes("shadowcatcher", 65, 33), 3),
     "textured": (lambda: scenes.textured_room_scene(width=129, height=71, textured_light=True), 3),
+    "textured_few": (lambda: scenes.textured_room_scene(width=100, height=100), 1),         # too few paths
+    "textured_enough": (lambda: scenes.textured_room_scene(width=100, height=100), 2),
     "lens": (lambda: _camera(scenes.room_scene(width=64, height=36), lens_radius=0.1, focal_length=3.0), 2),
     "env_camera": (lambda: _camera(scenes.room_scene(width=64, height=36), type="env"), 2),
     "batches": (lambda: scenes.room_scene(width=1500, height=1501, bounces=2), 3),         # one frame a batch

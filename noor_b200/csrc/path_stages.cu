@@ -115,7 +115,9 @@ constexpr uint32_t kStageMaxPaths = 1u << 22;
 // 161 us, sky 166 / 127).
 constexpr uint64_t kStageMinBumpPaths = 20000;
 
-// the batch's buffers, laid out in one allocation that the context keeps.
+// the batch's buffers, laid out in one allocation that the context keeps, from
+// the device's pool: a new context takes over what an earlier one gave back
+// (cudaMalloc was half of its first 256x256 frame, 0.3 of 0.6 ms).
 // False (nothing changed) where the device has no room for it.
 static bool stage_buffers(Context& C, uint32_t paths, uint32_t frames, uint32_t bounces, bool diff, StageDev& W) {
     size_t at = 0;
@@ -131,10 +133,10 @@ static bool stage_buffers(Context& C, uint32_t paths, uint32_t frames, uint32_t 
                  df = place(diff ? 64 * n : 0), cnt = place(4 * (size_t)kStWords * (bounces + 1)),
                  first = place(16 * (size_t)frames);
     if (C.stage_bytes < at) {
-        if (C.stage_buf) cudaFree(C.stage_buf);
+        if (C.stage_buf) cudaFreeAsync(C.stage_buf, C.stream);
         C.stage_buf = nullptr;
         C.stage_bytes = 0;
-        if (cudaMalloc(&C.stage_buf, at) != cudaSuccess) {
+        if (cudaMallocAsync(&C.stage_buf, at, C.stream) != cudaSuccess) {
             cudaGetLastError();
             C.stage_buf = nullptr;
             return false;

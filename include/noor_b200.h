@@ -377,6 +377,15 @@ int noor_abi_sizes(uint32_t* out, int n);
  * frames beyond that, or without the memory for it, take the megakernel (the
  * same film). */
 int noor_render_frames(unsigned int* frame_count, unsigned int n_frames);
+/* Which kernels the current context renders its frames and its adjoint with,
+ * to compare them with each other: by default (AUTO) the library chooses by
+ * the size of the work.  The results are the same.  A route that cannot serve
+ * a call (no memory for the stages) leaves it to the library's choice.
+ * frames: AUTO, MEGAKERNEL or STAGED; adjoint: AUTO, REPLAY (a thread per
+ * path) or STAGED. */
+enum { NOOR_ROUTE_AUTO = 0, NOOR_ROUTE_MEGAKERNEL = 1, NOOR_ROUTE_STAGED = 2 };
+enum { NOOR_ROUTE_REPLAY = NOOR_ROUTE_MEGAKERNEL };
+int noor_route(int frames, int adjoint);
 /* Film readback: rgba = mean of the folded samples (w = 1). */
 int noor_get_framebuffer(float* host_rgba, size_t n_pixels);
 int noor_get_framebuffer_device(float* device_rgba, size_t n_pixels);

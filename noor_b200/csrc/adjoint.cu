@@ -392,7 +392,9 @@ static int adjoint_run(const noor_adjoint_desc* desc, int mode, float* image, co
     P.frame0 = desc->first_frame ? desc->first_frame : 1;
     P.status = C->status;
     bool staged = false;
-    if ((rc = adjoint_staged(*C, S, P, mode, image, &staged)) || staged) return rc;
+    if (C->adjoint_route != NOOR_ROUTE_REPLAY &&
+        ((rc = adjoint_staged(*C, S, P, mode, image, &staged)) || staged))
+        return rc;
     const uint32_t npix = C->cam.w * C->cam.h;
     const size_t sm = (size_t)S.stack_words * kAdjBlock * 4;
     // buffers: per-sample radiance of one chunk, and (forward) the Kahan

@@ -699,7 +699,7 @@ int render_frames(Context& C, uint32_t frame0, uint32_t n) {
     a.status = C.status;
     a.counters = C.counters;
     bool staged = false;
-    if ((rc = render_staged(C, st.dev, a, &staged))) return rc;
+    if (C.frames_route != NOOR_ROUTE_MEGAKERNEL && (rc = render_staged(C, st.dev, a, &staged))) return rc;
     if (!staged) {
         cudaError_t e = launch_megakernel(st.dev, C.cam, a, C.stream);
         if (e != cudaSuccess) return cuda_fail(e, "megakernel");
@@ -859,6 +859,17 @@ extern "C" int noor_render_frames(unsigned int* frame_count, unsigned int n_fram
     if ((rc = render_frames(*C, *frame_count, n_frames))) return rc;
     if ((rc = sync_and_check(*C, "noor_render_frames"))) return rc;
     *frame_count += n_frames;
+    return NOOR_OK;
+}
+
+extern "C" int noor_route(int frames, int adjoint) {
+    Context* C;
+    int rc = need_ctx(C);
+    if (rc) return rc;
+    for (int r : {frames, adjoint})
+        if (r < NOOR_ROUTE_AUTO || r > NOOR_ROUTE_STAGED) return set_error(NOOR_ERR_INVALID, "noor_route: unknown route");
+    C->frames_route = frames;
+    C->adjoint_route = adjoint;
     return NOOR_OK;
 }
 

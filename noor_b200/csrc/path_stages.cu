@@ -171,7 +171,7 @@ int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done) 
     *done = false;
     const uint64_t npix = (uint64_t)C.cam.w * C.cam.h;
     if (npix > kStageMaxPaths || S.bounces == 0 || S.bounces > 1024) return NOOR_OK;
-    if (S.has_bump && npix * a.nframes < kStageMinBumpPaths) return NOOR_OK;
+    if (S.has_bump && npix * a.nframes < kStageMinBumpPaths && C.frames_route != NOOR_ROUTE_STAGED) return NOOR_OK;
     const uint32_t nb = (uint32_t)std::min<uint64_t>(a.nframes, kStageMaxPaths / npix);
     StageDev W{};
     if (!stage_buffers(C, (uint32_t)npix * nb, nb, S.bounces, S.has_bump != 0u, W)) return NOOR_OK;

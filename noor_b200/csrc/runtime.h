@@ -78,6 +78,7 @@ struct Context {
     size_t adj_bytes = 0;
     void* stage_buf = nullptr;  // staged renderer: a batch's paths and queues
     size_t stage_bytes = 0;
+    int frames_route = 0, adjoint_route = 0;  // noor_route
     cudaEvent_t events[8] = {};
     uint64_t launches = 0;
     WavefrontState* wf = nullptr;

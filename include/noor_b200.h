@@ -373,17 +373,18 @@ int noor_abi_sizes(uint32_t* out, int n);
 
 /* Render frames *frame_count .. *frame_count+n_frames-1 (one path per (pixel,
  * frame)) and fold them into the film in frame order; *frame_count +=
- * n_frames.  Staged over the paths of up to 2^22 pixels x frames at a time;
- * frames beyond that, or without the memory for it, take the megakernel (the
- * same film). */
+ * n_frames.  Few paths are rendered in one launch with a thread each; more
+ * are staged, up to 2^22 pixels x frames at a time; frames beyond that, or
+ * without the memory for it, take the megakernel (the same film). */
 int noor_render_frames(unsigned int* frame_count, unsigned int n_frames);
 /* Which kernels the current context renders its frames and its adjoint with,
  * to compare them with each other: by default (AUTO) the library chooses by
  * the size of the work.  The results are the same.  A route that cannot serve
  * a call (no memory for the stages) leaves it to the library's choice.
- * frames: AUTO, MEGAKERNEL or STAGED; adjoint: AUTO, REPLAY (a thread per
+ * frames: AUTO, MEGAKERNEL, STAGED or SMALL (a thread per path, on the
+ * four-wide tree); adjoint: AUTO, REPLAY (a thread per
  * path) or STAGED. */
-enum { NOOR_ROUTE_AUTO = 0, NOOR_ROUTE_MEGAKERNEL = 1, NOOR_ROUTE_STAGED = 2 };
+enum { NOOR_ROUTE_AUTO = 0, NOOR_ROUTE_MEGAKERNEL = 1, NOOR_ROUTE_STAGED = 2, NOOR_ROUTE_SMALL = 3 };
 enum { NOOR_ROUTE_REPLAY = NOOR_ROUTE_MEGAKERNEL };
 int noor_route(int frames, int adjoint);
 /* Film readback: rgba = mean of the folded samples (w = 1). */

@@ -21,8 +21,9 @@ CSRC = PKG / "csrc"
 OUT = PKG / "libnoor_b200.so"
 OBJ = ROOT / "_build" / "noor_b200"
 
-CU_SOURCES = ["megakernel_wt.cu", "megakernel_wald.cu", "path_stages_wt.cu", "path_stages_wald.cu",
-              "path_stages.cu", "kernels.cu", "envmap.cu", "context.cu", "wavefront.cu", "adjoint.cu", "adjoint_stages.cu", "noalloc.cu", "tonemap.cu",
+CU_SOURCES = ["megakernel_wt.cu", "megakernel_wald.cu", "small_frames_wt.cu", "small_frames_wald.cu",
+              "path_stages_wt.cu", "path_stages_wald.cu", "path_stages.cu",
+              "kernels.cu", "envmap.cu", "context.cu", "wavefront.cu", "adjoint.cu", "adjoint_stages.cu", "noalloc.cu", "tonemap.cu",
               "bvh_gpu.cu"]
 # the GPU BVH builder rounds its split search as the host builder does
 CU_EXTRA = {"bvh_gpu.cu": ["-fmad=false"]}

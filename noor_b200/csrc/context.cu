@@ -669,8 +669,9 @@ int need_ctx(Context*& C) {
     return NOOR_OK;
 }
 
-// render frames [frame0, frame0 + n): staged (path_stages.cuh), or with the
-// megakernel where the staged renderer has no room for a frame's paths
+// render frames [frame0, frame0 + n): few paths with a thread each
+// (small_frames.cuh), else staged (path_stages.cuh), or with the megakernel
+// where the staged renderer has no room for a frame's paths
 int render_frames(Context& C, uint32_t frame0, uint32_t n) {
     if (n == 0) return NOOR_OK;
     if (frame0 == 0) return set_error(NOOR_ERR_INVALID, "frame numbers start at 1");
@@ -698,10 +699,15 @@ int render_frames(Context& C, uint32_t frame0, uint32_t n) {
     a.lookat = C.lookat;
     a.status = C.status;
     a.counters = C.counters;
+    const int route = C.frames_route;
+    const bool small = a.chunks == a.nframes &&  // a thread per path: every sample of a pixel is a chunk
+                       (route == NOOR_ROUTE_SMALL ||
+                        (route == NOOR_ROUTE_AUTO && small_frames_fit(st.dev, C.cam, a, C.sm_count)));
     bool staged = false;
-    if (C.frames_route != NOOR_ROUTE_MEGAKERNEL && (rc = render_staged(C, st.dev, a, &staged))) return rc;
+    if (!small && route != NOOR_ROUTE_MEGAKERNEL && (rc = render_staged(C, st.dev, a, &staged))) return rc;
     if (!staged) {
-        cudaError_t e = launch_megakernel(st.dev, C.cam, a, C.stream);
+        const cudaError_t e = small ? launch_small_frames(st.dev, C.cam, a, C.sm_count, C.stream)
+                                    : launch_megakernel(st.dev, C.cam, a, C.stream);
         if (e != cudaSuccess) return cuda_fail(e, "megakernel");
         C.launches += chunks > 1 ? 2 : 1;
     }
@@ -866,8 +872,8 @@ extern "C" int noor_route(int frames, int adjoint) {
     Context* C;
     int rc = need_ctx(C);
     if (rc) return rc;
-    for (int r : {frames, adjoint})
-        if (r < NOOR_ROUTE_AUTO || r > NOOR_ROUTE_STAGED) return set_error(NOOR_ERR_INVALID, "noor_route: unknown route");
+    if (frames < NOOR_ROUTE_AUTO || frames > NOOR_ROUTE_SMALL || adjoint < NOOR_ROUTE_AUTO || adjoint > NOOR_ROUTE_STAGED)
+        return set_error(NOOR_ERR_INVALID, "noor_route: unknown route");
     C->frames_route = frames;
     C->adjoint_route = adjoint;
     return NOOR_OK;

@@ -498,13 +498,32 @@ NB_D void make_isect(const DevScene& S, const float3& o, const float3& d, float 
     if (to) I.uv = to->uv;
 }
 
+// pixel of the q-th pixel slot: 8x4 tiles in row-major order, row-major inside
+// a tile, so that a warp's camera rays form a compact bundle; pixels outside
+// the whole tiles follow row by row (the right strip, then the bottom rows)
+NB_D uint32_t stage_pixel(uint32_t q, uint32_t w, uint32_t h) {
+    const uint32_t w8 = w & ~7u, h4 = h & ~3u;
+    const uint32_t full = w8 * h4;
+    if (q < full) {
+        const uint32_t t = q >> 5, r = q & 31u;
+        const uint32_t tx = t % (w8 >> 3), ty = t / (w8 >> 3);
+        return (ty * 4u + (r >> 3)) * w + tx * 8u + (r & 7u);
+    }
+    q -= full;
+    const uint32_t rw = w - w8;
+    if (q < rw * h4) return (q / rw) * w + w8 + q % rw;
+    q -= rw * h4;
+    return (h4 + q / w) * w + q % w;
+}
+
 // pathtracer() of noor/cuda/path_tracer.cu:26-75; returns clamp(L, 0, 100)
 // EXT false: the specialisation for scenes whose materials use only the
 // Lambert, conductor and Fresnel-specular lobes
 // DIFF: the specialisation for scenes with bump maps, whose rays carry
 // differentials (rd: the camera ray's) -- the reference bumps only where a
 // differential ray arrives (accumulate.cuh:90-92)
-template <int ISECT, bool EXT = true, bool DIFF = false>
+// WIDE: the walks take the four-wide tree
+template <int ISECT, bool EXT = true, bool DIFF = false, bool WIDE = false>
 NB_D float3 path_radiance(const DevScene& S, float3 o, float3 d, Rng& rng, const SmemStack& st, uint32_t* status,
                           RayStats& rs, float3* first_hit, bool* first_hit_valid, RayDiff rd = RayDiff{}) {
     float3 L = f3(0.0f);
@@ -514,7 +533,7 @@ NB_D float3 path_radiance(const DevScene& S, float3 o, float3 d, Rng& rng, const
         float tmax = kInf;
         HitRec rec;
         rs.ext++;
-        if (!trace_closest<ISECT, EXT>(S, o, d, tmax, rec, st, status)) {
+        if (!trace_primary<ISECT, EXT, WIDE>(S, HeldRay{o, d}, tmax, rec, st, status)) {
             if (S.sky_on && (bounce == 0 || spec_bounce)) L += beta * env_eval<EXT>(S, normalize_fast(d));
             break;
         }
@@ -553,13 +572,13 @@ NB_D float3 path_radiance(const DevScene& S, float3 o, float3 d, Rng& rng, const
         float3 Ld = light_sample_contrib<EXT>(S, m, I, rng, S.mis != 0, li, picked, sr);
         if (!is_black(Ld)) {
             rs.shadow++;
-            if (trace_any<ISECT, EXT>(S, sr.o, sr.d, sr.tmax, st, status)) Ld = f3(0.0f);
+            if (trace_shadow<ISECT, EXT, WIDE>(S, HeldRay{sr.o, sr.d}, sr.tmax, st, status)) Ld = f3(0.0f);
         }
         if (S.mis && picked) {
             float3 c = bsdf_mis_contrib<EXT>(S, m, I, rng, li, sr);
             if (!is_black(c)) {
                 rs.shadow++;
-                if (trace_any<ISECT, EXT>(S, sr.o, sr.d, sr.tmax, st, status)) c = f3(0.0f);
+                if (trace_shadow<ISECT, EXT, WIDE>(S, HeldRay{sr.o, sr.d}, sr.tmax, st, status)) c = f3(0.0f);
             }
             Ld += c;
         }

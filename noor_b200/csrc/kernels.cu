@@ -228,16 +228,57 @@ __global__ void k_debug_skydome(DevScene S, DevCamera C, uint32_t frame, float4*
 }
 
 // ------------------------------------------------------------ launchers
+static cudaError_t launch_fold(const DevCamera& C, const MegaArgs& a, cudaStream_t s) {
+    if (a.chunks <= 1u) return cudaSuccess;
+    const uint32_t npix = C.w * C.h;
+    fold_partials<<<(npix + 255) / 256, 256, 0, s>>>(npix, a.chunks, a.fresh, a.film_sum, a.film_comp, a.part_sum,
+                                                      a.part_comp);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_megakernel(const DevScene& S, const DevCamera& C, const MegaArgs& a, cudaStream_t s) {
-    cudaError_t e = S.isect == NOOR_ISECT_WATERTIGHT ? launch_megakernel_wt(S, C, a, s) : launch_megakernel_wald(S, C, a, s);
-    if (e != cudaSuccess) return e;
-    if (a.chunks > 1u) {
-        const uint32_t npix = C.w * C.h;
-        fold_partials<<<(npix + 255) / 256, 256, 0, s>>>(npix, a.chunks, a.fresh, a.film_sum, a.film_comp,
-                                                          a.part_sum, a.part_comp);
-        e = cudaGetLastError();
-    }
-    return e;
+    const cudaError_t e =
+        S.isect == NOOR_ISECT_WATERTIGHT ? launch_megakernel_wt(S, C, a, s) : launch_megakernel_wald(S, C, a, s);
+    return e == cudaSuccess ? launch_fold(C, a, s) : e;
+}
+
+// The line between small frames (a thread per path) and the staged renderer.
+// A staged bounce costs its longest walk and two launches whatever the frame,
+// so the line rises with the bounces that a path can make and with the depth of
+// the tree; beyond it the stages' fuller warps win.  In waves of resident
+// threads, megakernel / stages / small frames in us:
+//   1.5   36-triangle room, 384x288: 2 bounces 140 / 134 / 108, 8: 362 / 323 / 307
+//         (448x336: 158 / 138 / 125 and 423 / 324 / 391); 2 bounces under the
+//         sky, 384x288: 280 / 227 / 212 and 333 / 242 / 242 (448x336: 383 / 250 / 320)
+//   4     8 bounces under the sky, 641x359: 164 k triangles 450 / 488 / 365 and
+//         608 / 497 / 492, 2.6 M triangles 774 / 718 / 540 (800x450: 651 / 497 / 545,
+//         851 / 816 / 664)
+//   1     with the code of all lights, textures and bump maps, 5 bounces in the
+//         textured room: 192x144 329 / 291 / 271, 320x240 514 / 371 / 403
+bool small_frames_fit(const DevScene& S, const DevCamera& C, const MegaArgs& a, int sm_count) {
+    const bool ext = ext_kernels(S, C), shallow = S.num_tris < 16384u;
+    const uint64_t wave = (uint64_t)sm_count * kSmallBlocks(ext) * kMegaBlock;
+    const uint64_t half_waves = ext ? 2 : (shallow || S.bounces < 4u) ? 3 : S.bounces < 6u ? 4 : 8;
+    return 2 * (uint64_t)C.w * C.h * a.nframes <= wave * half_waves;
+}
+
+cudaError_t launch_small_frames(const DevScene& S, const DevCamera& C, const MegaArgs& a, int sm_count, cudaStream_t s) {
+    // trees without a four-wide form: the megakernel's walks
+    if (!S.mega4) return launch_megakernel(S, C, a, s);
+    // Paths a warp, a power of two: 32, or fewer where that leaves warps to
+    // spare.  Walks fill the resident warps (one frame under the sky of 97x61,
+    // 32 / 8 / 4 paths a warp: 147 / 115 / 102 us); the larger code of the
+    // other lights and textures is bound by its instruction fetch from some
+    // five warps per SM on (the textured room, 97x61: 130 / 107 / 128; 160x120,
+    // 32 / 16: 161 / 183).
+    const bool ext = ext_kernels(S, C);
+    const uint64_t warps = (uint64_t)sm_count * (ext ? 5 : kSmallBlocks(ext) * (kMegaBlock / 32));
+    const uint64_t paths = (uint64_t)C.w * C.h * a.nframes;
+    uint32_t lanes = 32;
+    while (lanes > 1u && paths <= warps * (lanes / 2)) lanes /= 2;
+    const cudaError_t e = S.isect == NOOR_ISECT_WATERTIGHT ? launch_small_frames_wt(S, C, a, lanes, s)
+                                                           : launch_small_frames_wald(S, C, a, lanes, s);
+    return e == cudaSuccess ? launch_fold(C, a, s) : e;
 }
 
 cudaError_t launch_resolve(uint32_t npix, int mode, float inv_count, const float4* film_sum, float4* out,

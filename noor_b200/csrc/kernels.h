@@ -6,6 +6,14 @@ namespace nb {
 
 constexpr int kMegaBlock = 128;
 constexpr int kTraceBlock = 128;
+// resident blocks per SM of the small frames' kernel
+constexpr int kSmallBlocks(bool ext) { return ext ? 3 : 4; }
+// whether a scene seen through a camera needs the kernels with the code of
+// every lobe, light shape, camera and texture
+inline bool ext_kernels(const DevScene& S, const DevCamera& C) {
+    return S.has_bump || S.ext_lobes || S.ext_lights || S.env_ref || S.has_tex || C.type != NOOR_CAMERA_PERSP ||
+           C.lens_radius > 0.0f;
+}
 
 struct MegaArgs {
     uint32_t frame0;        // RNG frame number of the first sample
@@ -25,6 +33,14 @@ cudaError_t launch_megakernel(const DevScene& S, const DevCamera& C, const MegaA
 // ... its render kernel, per intersector
 cudaError_t launch_megakernel_wt(const DevScene& S, const DevCamera& C, const MegaArgs& a, cudaStream_t s);
 cudaError_t launch_megakernel_wald(const DevScene& S, const DevCamera& C, const MegaArgs& a, cudaStream_t s);
+// Frames of few paths (small_frames.cuh): whether a thread per path renders
+// them soonest, and the launch (chunks = nframes)
+bool small_frames_fit(const DevScene& S, const DevCamera& C, const MegaArgs& a, int sm_count);
+cudaError_t launch_small_frames(const DevScene& S, const DevCamera& C, const MegaArgs& a, int sm_count, cudaStream_t s);
+cudaError_t launch_small_frames_wt(const DevScene& S, const DevCamera& C, const MegaArgs& a, uint32_t lanes,
+                                   cudaStream_t s);
+cudaError_t launch_small_frames_wald(const DevScene& S, const DevCamera& C, const MegaArgs& a, uint32_t lanes,
+                                     cudaStream_t s);
 cudaError_t launch_resolve(uint32_t npix, int mode, float inv_count, const float4* film_sum, float4* out,
                            cudaStream_t s);
 cudaError_t launch_trace_closest(const DevScene& S, const noor_ray* rays, noor_hit* hits, size_t n, uint32_t* status,

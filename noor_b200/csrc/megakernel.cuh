@@ -111,8 +111,7 @@ cudaError_t launch_megakernel_isect(const DevScene& S, const DevCamera& C, const
     const uint64_t threads = (uint64_t)C.w * C.h * a.chunks;
     const uint32_t grid = (uint32_t)((threads + kMegaBlock - 1) / kMegaBlock);
     const size_t sm = (size_t)S.stack_cap * kMegaBlock * sizeof(uint32_t);
-    const bool ext_cam = C.type != NOOR_CAMERA_PERSP || C.lens_radius > 0.0f;
-    const bool ext = S.ext_lobes || S.ext_lights || S.env_ref || S.has_tex || ext_cam;
+    const bool ext = ext_kernels(S, C);
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;

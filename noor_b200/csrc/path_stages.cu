@@ -106,15 +106,6 @@ __global__ void __launch_bounds__(256) st_fold(DevCamera C, StageDev W, StageFol
 // paths a batch holds at most: 228 bytes of state each (64 more with bump
 // maps), a gigabyte in all; a frame beyond it is left to the megakernel
 constexpr uint32_t kStageMaxPaths = 1u << 22;
-// Scenes with bump maps: fewer paths than this go to the megakernel.  The
-// stages store and load 64 bytes of differentials a bounce and run the largest
-// shading kernel, and below one path a lane the megakernel's latency is the
-// shorter one (one sample of the textured room, megakernel / staged:
-// 128x96 238 / 260 us, 160x120 255 / 274, 192x144 330 / 298); scenes without
-// are at least as fast staged from the smallest frames on (97x61 room 181 /
-// 161 us, sky 166 / 127).
-constexpr uint64_t kStageMinBumpPaths = 20000;
-
 // the batch's buffers, laid out in one allocation that the context keeps, from
 // the device's pool: a new context takes over what an earlier one gave back
 // (cudaMalloc was half of its first 256x256 frame, 0.3 of 0.6 ms).
@@ -171,7 +162,6 @@ int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done) 
     *done = false;
     const uint64_t npix = (uint64_t)C.cam.w * C.cam.h;
     if (npix > kStageMaxPaths || S.bounces == 0 || S.bounces > 1024) return NOOR_OK;
-    if (S.has_bump && npix * a.nframes < kStageMinBumpPaths && C.frames_route != NOOR_ROUTE_STAGED) return NOOR_OK;
     const uint32_t nb = (uint32_t)std::min<uint64_t>(a.nframes, kStageMaxPaths / npix);
     StageDev W{};
     if (!stage_buffers(C, (uint32_t)npix * nb, nb, S.bounces, S.has_bump != 0u, W)) return NOOR_OK;

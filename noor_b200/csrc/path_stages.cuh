@@ -23,12 +23,10 @@
 // the stages run 13 and more lanes of small kernels.  Measured against the
 // megakernel: 256x256 room 0.305 -> 0.248 ms, 1920x1080 of a 2.6M-triangle
 // sky scene 3.68 -> 2.45, sixteen 960x540 frames of an environment-lit field
-// 14.7 -> 4.06, four 641x359 frames of the textured room 3.98 -> 0.88.  Small
-// frames are bound by latency, bounce after bounce: the stages are launched
-// ahead of each other's end and a bounce with few paths costs its longest walk
-// (one sample, 128x96 room 196 -> 172 us, 97x61 sky of 8 spheres 166 -> 127;
-// against it, 192x144 of a 1.3M-triangle sky 307 -> 352 for one camera of four,
-// whose longest walks fall on different paths in each bounce).
+// 14.7 -> 4.06, four 641x359 frames of the textured room 3.98 -> 0.88.  Few
+// paths are bound by latency, bounce after bounce: the stages are launched
+// ahead of each other's end, and a bounce costs its longest walk, which falls on
+// another path each time.  small_frames.cuh renders those frames.
 #pragma once
 #include "integrator.cuh"
 #include "kernels.h"
@@ -91,24 +89,6 @@ struct StageFold {
     float4* part_comp;
     float4* lookat;
 };
-
-// pixel of the q-th pixel slot: 8x4 tiles in row-major order, row-major inside
-// a tile, so that a warp's camera rays form a compact bundle; pixels outside
-// the whole tiles follow row by row (the right strip, then the bottom rows)
-NB_D uint32_t stage_pixel(uint32_t q, uint32_t w, uint32_t h) {
-    const uint32_t w8 = w & ~7u, h4 = h & ~3u;
-    const uint32_t full = w8 * h4;
-    if (q < full) {
-        const uint32_t t = q >> 5, r = q & 31u;
-        const uint32_t tx = t % (w8 >> 3), ty = t / (w8 >> 3);
-        return (ty * 4u + (r >> 3)) * w + tx * 8u + (r & 7u);
-    }
-    q -= full;
-    const uint32_t rw = w - w8;
-    if (q < rw * h4) return (q / rw) * w + w8 + q % rw;
-    q -= rw * h4;
-    return (h4 + q / w) * w + q % w;
-}
 
 // warp-aggregated push: lanes of one warp may push onto different queues
 NB_D uint32_t stage_push(uint32_t* counter) {

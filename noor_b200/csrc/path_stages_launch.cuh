@@ -37,9 +37,8 @@ cudaError_t run_stages(const DevScene& S, const DevCamera& C, const StageDev& W,
 template <int ISECT>
 cudaError_t launch_stages(const DevScene& S, const DevCamera& C, const StageDev& W, int sm_count, uint64_t* launches,
                           cudaStream_t s) {
-    const bool ext_cam = C.type != NOOR_CAMERA_PERSP || C.lens_radius > 0.0f;
     if (S.has_bump) return run_stages<ISECT, true, true>(S, C, W, sm_count, launches, s);
-    if (S.ext_lobes || S.ext_lights || S.env_ref || S.has_tex || ext_cam)
+    if (ext_kernels(S, C))
         return run_stages<ISECT, true, false>(S, C, W, sm_count, launches, s);
     return run_stages<ISECT, false, false>(S, C, W, sm_count, launches, s);
 }

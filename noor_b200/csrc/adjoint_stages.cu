@@ -198,14 +198,18 @@ __global__ void __launch_bounds__(128, 4) adj_shade(DevScene S, AdjParams P, Adj
         const int nt = queued_terms<ISECT>(S, P, W, cnt, i, m0, me, I, rng, T, dir);
         uint32_t word = I.mat;
         for (int k = 0; k < nt; ++k) {
-            const float3 v = T[k].X * T[k].f.f;
-            W.pend[2 * r + k] = make_float4(v.x, v.y, v.z, T[k].s);
+            // (a scale of zero goes into the product: zero marks an occluded term)
+            const bool zero = T[k].s == 0.0f;
+            float3 v = T[k].X * T[k].f.f;
+            if (zero) v = v * T[k].s;
+            W.pend[2 * r + k] = make_float4(v.x, v.y, v.z, zero ? 1.0f : T[k].s);
             if (RECORD) {
                 record_term(A, r, k, T[k], dir[k]);
                 if (T[k].env) word |= kAdjEnv << k;
             }
         }
         const bool pend = nt > 0;
+        if (!pend) L += beta * 0.0f;  // as the replay, where the throughput is not finite
         if (pend || RECORD) {
             for (int k = nt; k < 2; ++k) W.pend[2 * r + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             W.pbeta[r] = make_float4(beta.x, beta.y, beta.z, 0.0f);

@@ -290,6 +290,8 @@ __global__ void __launch_bounds__(128, EXT ? 4 : 6) st_shade(DevScene S, StageDe
             W.pend[2 * i] = make_float4(c0.x, c0.y, c0.z, has0 ? 1.0f : 0.0f);
             W.pend[2 * i + 1] = make_float4(c1.x, c1.y, c1.z, has1 ? 1.0f : 0.0f);
             W.pbeta[i] = make_float4(beta.x, beta.y, beta.z, 0.0f);
+        } else {
+            L += beta * 0.0f;  // as the megakernel: a throughput that is not finite ends the sample's radiance
         }
         rng.next();
         rng.next();

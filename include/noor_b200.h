@@ -377,6 +377,15 @@ int noor_abi_sizes(uint32_t* out, int n);
  * are staged, up to 2^22 pixels x frames at a time; frames beyond that, or
  * without the memory for it, take the megakernel (the same film). */
 int noor_render_frames(unsigned int* frame_count, unsigned int n_frames);
+/* What the context keeps on the device for the paths of a call, of which each
+ * of the two below takes at most `bytes` from now on (by default all of it):
+ * the staged renderer 228 bytes a path (292 with bump maps), for at most 2^22
+ * paths at a time; the adjoint 244 bytes a path forward and 184 + 148 per bounce
+ * of the limit backward, for at most 2^21 paths and 4 GiB at a time (1.6 GB for
+ * 512 x 512 pixels, 16 samples and 4 bounces).  With less, or where the device
+ * has no more, they take fewer frames or samples at a time, and where one does
+ * not fit, the kernels that need no such memory. */
+int noor_workspace_limit(size_t bytes);
 /* Which kernels the current context renders its frames and its adjoint with,
  * to compare them with each other: by default (AUTO) the library chooses by
  * the size of the work.  The results are the same.  A route that cannot serve

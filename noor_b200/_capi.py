@@ -223,6 +223,7 @@ PROTOTYPES = {
     "noor_tonemap_device": (C.c_int, [C.c_void_p, C.c_size_t, C.c_int, C.c_float, C.c_void_p]),
     "noor_save_image": (C.c_int, [C.c_char_p, C.c_int, C.c_float]),
     "noor_render_frames": (C.c_int, [C.POINTER(C.c_uint), C.c_uint]),
+    "noor_workspace_limit": (C.c_int, [C.c_size_t]),
     "noor_route": (C.c_int, [C.c_int, C.c_int]),
     "noor_get_framebuffer": (C.c_int, [pf, C.c_size_t]),
     "noor_get_framebuffer_device": (C.c_int, [C.c_void_p, C.c_size_t]),

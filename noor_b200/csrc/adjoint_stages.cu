@@ -420,32 +420,36 @@ static int run_staged(Context& C, const DevScene& S, const AdjParams& P, int mod
     const size_t per_path = 180 + 48 * (size_t)verts + (record ? 100 * (size_t)verts + 4 : 16);
     const size_t most = std::min<size_t>(kAdjStagePaths, kAdjStageBytes / per_path);
     if (npix > most) return NOOR_OK;
-    const uint32_t chunk = std::min<uint32_t>(P.spp, (uint32_t)(most / npix));
-    const size_t n = (size_t)npix * chunk;
-    size_t at = 0;
+    // samples a chunk, halved until the device has room and the context's limit allows
+    uint32_t chunk = std::min<uint32_t>(P.spp, (uint32_t)(most / npix));
+    size_t n, at, o, d, beta, L, hit, hit2, q0, q1, qs, qsh, sho, shd, pend, pbeta, ta, te, td, sc, vw, nv, lb, kh, cnt, first;
     auto place = [&](size_t bytes) {
         const size_t p = at;
         at += (bytes + 255) & ~(size_t)255;
         return p;
     };
-    const size_t o = place(16 * n), d = place(16 * n), beta = place(16 * n), L = place(16 * n), hit = place(16 * n),
-                 hit2 = place(8 * n), q0 = place(4 * n), q1 = place(4 * n), qs = place(4 * n * kStageKinds),
-                 qsh = place(8 * n), sho = place(32 * n), shd = place(32 * n), pend = place(32 * n * verts),
-                 pbeta = place(16 * n * verts), ta = place(record ? 32 * n * verts : 0),
-                 te = place(record ? 32 * n * verts : 0), td = place(record ? 16 * n * verts : 0),
-                 sc = place(record ? 16 * n * verts : 0), vw = place(record ? 4 * n * verts : 0),
-                 nv = place(record ? 4 * n : 0), lb = place(record ? 0 : 16 * n), kh = place(record ? 0 : 32 * (size_t)npix),
-                 cnt = place(4 * (size_t)kStWords * (S.bounces + 1)), first = place(16 * (size_t)chunk);
-    if (C.adj_bytes < at) {
+    for (;; chunk /= 2) {
+        if (chunk == 0) return NOOR_OK;
+        n = (size_t)npix * chunk;
+        at = 0;
+        o = place(16 * n), d = place(16 * n), beta = place(16 * n), L = place(16 * n), hit = place(16 * n);
+        hit2 = place(8 * n), q0 = place(4 * n), q1 = place(4 * n), qs = place(4 * n * kStageKinds), qsh = place(8 * n);
+        sho = place(32 * n), shd = place(32 * n), pend = place(32 * n * verts), pbeta = place(16 * n * verts);
+        ta = place(record ? 32 * n * verts : 0), te = place(record ? 32 * n * verts : 0);
+        td = place(record ? 16 * n * verts : 0), sc = place(record ? 16 * n * verts : 0);
+        vw = place(record ? 4 * n * verts : 0), nv = place(record ? 4 * n : 0);
+        lb = place(record ? 0 : 16 * n), kh = place(record ? 0 : 32 * (size_t)npix);
+        cnt = place(4 * (size_t)kStWords * (S.bounces + 1)), first = place(16 * (size_t)chunk);
+        if (at <= C.adj_bytes) break;
+        if (at > C.workspace_limit) continue;
         if (C.adj_buf) cudaFree(C.adj_buf);
-        C.adj_buf = nullptr;
         C.adj_bytes = 0;
-        if (cudaMalloc(&C.adj_buf, at) != cudaSuccess) {
-            cudaGetLastError();
-            C.adj_buf = nullptr;
-            return NOOR_OK;
+        if (cudaMalloc(&C.adj_buf, at) == cudaSuccess) {
+            C.adj_bytes = at;
+            break;
         }
-        C.adj_bytes = at;
+        cudaGetLastError();
+        C.adj_buf = nullptr;
     }
     char* p = static_cast<char*>(C.adj_buf);
     AdjStage A{};

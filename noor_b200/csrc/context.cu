@@ -868,6 +868,24 @@ extern "C" int noor_render_frames(unsigned int* frame_count, unsigned int n_fram
     return NOOR_OK;
 }
 
+extern "C" int noor_workspace_limit(size_t bytes) {
+    Context* C;
+    int rc = need_ctx(C);
+    if (rc) return rc;
+    C->workspace_limit = bytes;
+    if (C->stage_bytes > bytes) {
+        cudaFreeAsync(C->stage_buf, C->stream);
+        C->stage_buf = nullptr;
+        C->stage_bytes = 0;
+    }
+    if (C->adj_bytes > bytes) {
+        cudaFree(C->adj_buf);
+        C->adj_buf = nullptr;
+        C->adj_bytes = 0;
+    }
+    return sync_and_check(*C, "noor_workspace_limit");
+}
+
 extern "C" int noor_route(int frames, int adjoint) {
     Context* C;
     int rc = need_ctx(C);

@@ -106,33 +106,39 @@ __global__ void __launch_bounds__(256) st_fold(DevCamera C, StageDev W, StageFol
 // paths a batch holds at most: 228 bytes of state each (64 more with bump
 // maps), a gigabyte in all; a frame beyond it is left to the megakernel
 constexpr uint32_t kStageMaxPaths = 1u << 22;
-// the batch's buffers, laid out in one allocation that the context keeps, from
-// the device's pool: a new context takes over what an earlier one gave back
-// (cudaMalloc was half of its first 256x256 frame, 0.3 of 0.6 ms).
-// False (nothing changed) where the device has no room for it.
-static bool stage_buffers(Context& C, uint32_t paths, uint32_t frames, uint32_t bounces, bool diff, StageDev& W) {
-    size_t at = 0;
+
+// The buffers of batches of `frames` frames, or of the most frames below that
+// (halved at each try) that the device has room for and the context's limit
+// allows, laid out in one allocation that the context keeps; stream-ordered, so
+// that a larger one takes over what is given back for it (a first 256x256 frame
+// 0.62 ms with cudaMalloc, 0.29 from a pool that holds memory).  Returns the
+// frames; 0 where there is no room for one.
+static uint32_t stage_buffers(Context& C, uint32_t npix, uint32_t frames, uint32_t bounces, bool diff, StageDev& W) {
+    size_t at, o, d, beta, L, pend, pbeta, hit, hit2, q0, q1, qshade, qshadow, sho, shd, df, cnt, first;
     auto place = [&](size_t bytes) {
         const size_t p = at;
         at += (bytes + 255) & ~(size_t)255;
         return p;
     };
-    const size_t n = paths;
-    const size_t o = place(16 * n), d = place(16 * n), beta = place(16 * n), L = place(16 * n), pend = place(32 * n),
-                 pbeta = place(16 * n), hit = place(16 * n), hit2 = place(8 * n), q0 = place(4 * n), q1 = place(4 * n),
-                 qshade = place(4 * n * kStageKinds), qshadow = place(8 * n), sho = place(32 * n), shd = place(32 * n),
-                 df = place(diff ? 64 * n : 0), cnt = place(4 * (size_t)kStWords * (bounces + 1)),
-                 first = place(16 * (size_t)frames);
-    if (C.stage_bytes < at) {
+    for (;; frames /= 2) {
+        if (frames == 0) return 0;
+        const size_t n = (size_t)npix * frames;
+        at = 0;
+        o = place(16 * n), d = place(16 * n), beta = place(16 * n), L = place(16 * n), pend = place(32 * n);
+        pbeta = place(16 * n), hit = place(16 * n), hit2 = place(8 * n), q0 = place(4 * n), q1 = place(4 * n);
+        qshade = place(4 * n * kStageKinds), qshadow = place(8 * n), sho = place(32 * n), shd = place(32 * n);
+        df = place(diff ? 64 * n : 0), cnt = place(4 * (size_t)kStWords * (bounces + 1));
+        first = place(16 * (size_t)frames);
+        if (at <= C.stage_bytes) break;
+        if (at > C.workspace_limit) continue;
         if (C.stage_buf) cudaFreeAsync(C.stage_buf, C.stream);
-        C.stage_buf = nullptr;
         C.stage_bytes = 0;
-        if (cudaMallocAsync(&C.stage_buf, at, C.stream) != cudaSuccess) {
-            cudaGetLastError();
-            C.stage_buf = nullptr;
-            return false;
+        if (cudaMallocAsync(&C.stage_buf, at, C.stream) == cudaSuccess) {
+            C.stage_bytes = at;
+            break;
         }
-        C.stage_bytes = at;
+        cudaGetLastError();
+        C.stage_buf = nullptr;
     }
     char* p = static_cast<char*>(C.stage_buf);
     W.o = (float4*)(p + o);
@@ -152,8 +158,8 @@ static bool stage_buffers(Context& C, uint32_t paths, uint32_t frames, uint32_t 
     W.sh_d = (float4*)(p + shd);
     W.count = (uint32_t*)(p + cnt);
     W.first = (float4*)(p + first);
-    W.cap = paths;
-    return true;
+    W.cap = npix * frames;
+    return frames;
 }
 
 // Frames a.frame0 .. + a.nframes - 1 into the film, staged.  *done = false
@@ -162,9 +168,10 @@ int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done) 
     *done = false;
     const uint64_t npix = (uint64_t)C.cam.w * C.cam.h;
     if (npix > kStageMaxPaths || S.bounces == 0 || S.bounces > 1024) return NOOR_OK;
-    const uint32_t nb = (uint32_t)std::min<uint64_t>(a.nframes, kStageMaxPaths / npix);
     StageDev W{};
-    if (!stage_buffers(C, (uint32_t)npix * nb, nb, S.bounces, S.has_bump != 0u, W)) return NOOR_OK;
+    const uint32_t nb = stage_buffers(C, (uint32_t)npix, (uint32_t)std::min<uint64_t>(a.nframes, kStageMaxPaths / npix),
+                                      S.bounces, S.has_bump != 0u, W);
+    if (nb == 0) return NOOR_OK;
     W.status = C.status;
     W.counters = C.counters;
     for (uint32_t f = 0; f < a.nframes; f += nb) {

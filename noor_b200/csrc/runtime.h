@@ -74,10 +74,11 @@ struct Context {
     uint32_t* status = nullptr;
     unsigned long long* counters = nullptr;
     void* scratch = nullptr;
-    void* adj_buf = nullptr;  // adjoint: per-sample radiance of one chunk + the forward's Kahan state
+    void* adj_buf = nullptr;  // adjoint: a chunk's paths, queues and records, or the replay's radiance
     size_t adj_bytes = 0;
     void* stage_buf = nullptr;  // staged renderer: a batch's paths and queues
     size_t stage_bytes = 0;
+    size_t workspace_limit = ~(size_t)0;  // of stage_buf and adj_buf each
     int frames_route = 0, adjoint_route = 0;  // noor_route
     cudaEvent_t events[8] = {};
     uint64_t launches = 0;

@@ -497,7 +497,18 @@ static int run_staged(Context& C, const DevScene& S, const AdjParams& P, int mod
         if (e != cudaSuccess) return cuda_fail(e, "adjoint");
         adj_begin<<<all, 256, 0, C.stream>>>(C.cam, A);
         adj_trace<ISECT><<<gt, trav, sm, C.stream>>>(S, C.cam, W, -1);
+        C.launches += 4;
         for (uint32_t b = 0; b < S.bounces; ++b) {
+            // every path may have ended long before the limit (kStageAsk)
+            if (b && b % kStageAsk == 0 && S.bounces - b >= kStageAsk) {
+                uint32_t left = 0;
+                if ((e = cudaMemcpyAsync(&left, W.count + b * kStWords + kStActive, 4, cudaMemcpyDeviceToHost,
+                                         C.stream)) ||
+                    (e = cudaStreamSynchronize(C.stream)))
+                    return cuda_fail(e, "adjoint");
+                if (left == 0) break;
+            }
+            C.launches += 2;
             if (record)
                 adj_shade<ISECT, true><<<gs, 128, 0, C.stream>>>(S, P, A, b);
             else
@@ -513,7 +524,6 @@ static int run_staged(Context& C, const DevScene& S, const AdjParams& P, int mod
                                1.0f / (float)P.spp, image, C.stream);
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "adjoint");
-        C.launches += 4 + 2 * (uint64_t)S.bounces;
     }
     *done = true;
     return sync_and_check(C, "adjoint");

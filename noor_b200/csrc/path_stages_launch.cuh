@@ -6,12 +6,6 @@
 
 namespace nb {
 
-// Every path may have ended long before the bounce limit, and a bounce without
-// paths takes 4 to 19 us (1920x1080 under the sky with a limit of 1024: 5.0 ms,
-// of which 4.4 for nothing).  So every kStageAsk bounces, where as many are to
-// come, the host asks what is left, which costs the launches' lead of some 20 us
-// (512x512 room, 9 bounces: 472 us, 491 with the asking).
-constexpr uint32_t kStageAsk = 8;
 constexpr int kStageTrav = 64, kStageTraceBlocks = 14;  // st_trace: 7 blocks of 128 threads in registers
 
 template <int ISECT, bool EXT, bool DIFF>

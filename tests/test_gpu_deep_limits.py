@@ -68,3 +68,35 @@ def test_launches_do_not_grow_with_the_limit(make):
         finally:
             r.close()
     assert n[1] <= n[0] <= 5 + 2 * 40
+
+
+def test_adjoint_launches_do_not_grow_with_the_limit():
+    import torch
+    from noor_b200.adjoint import _desc, scene_parameters
+    w, h, spp = 33, 17, 2
+    s = scenes.adjoint_scene(seed=5, width=w, height=h, spp=spp, bounces=1024, count=5, level=3, env_w=64, env_h=32)
+    r = scenes.Renderer(s)
+    alb, rough, env = scene_parameters(s)
+    gi = torch.ones((h, w, 3), device="cuda")
+    n, images, grads = [], [], []
+    try:
+        for bounces in (48, 1024):
+            d = _desc((w, h, spp, 1, bounces), alb, rough, env)
+            img = torch.zeros((h, w, 3), device="cuda")
+            g = [torch.zeros_like(t) for t in (alb, rough, env)]
+            torch.cuda.synchronize()
+            at = [C.c_uint64(), C.c_uint64()]
+            _capi.call("noor_launch_count", C.byref(at[0]))
+            _capi.call("noor_adjoint_forward", C.byref(d), C.c_void_p(img.data_ptr()))
+            _capi.call("noor_adjoint_backward", C.byref(d), C.c_void_p(gi.data_ptr()),
+                       *[C.c_void_p(t.data_ptr()) for t in g])
+            _capi.call("noor_launch_count", C.byref(at[1]))
+            n.append(at[1].value - at[0].value)
+            images.append(img)
+            grads.append(g)
+        assert n[1] == n[0] < 2 * (4 + 2 * 48)
+        assert torch.equal(images[0], images[1])
+        for x, y in zip(*grads):
+            assert float((x - y).norm()) <= 1e-5 * float(x.norm())
+    finally:
+        r.close()

@@ -38,6 +38,7 @@
 #include "bvh_gpu.h"
 #include "host_array.h"
 #include "host_common.h"
+#include "host_threads.h"
 
 namespace nbh {
 
@@ -282,30 +283,6 @@ static void parallel_for(uint32_t n, const F& f) {
             for (uint32_t i = b; i < e; ++i) f(i);
         });
     }
-    for (auto& th : pool) th.join();
-}
-
-// f(begin, end) over [0, n) in runs of 65536 and more, one per host thread;
-// where no thread can be had the caller does its run itself
-template <class F>
-static void parallel_ranges(size_t n, const F& f) {
-    const size_t nt = std::max<size_t>(1, std::min<size_t>(std::thread::hardware_concurrency(), n / 65536));
-    const size_t chunk = (n + nt - 1) / nt;
-    std::vector<std::thread> pool;
-    try {
-        pool.reserve(nt);
-    } catch (const std::bad_alloc&) {
-        return f(0, n);
-    }
-    for (size_t b = chunk; b < n; b += chunk) {
-        const size_t e = std::min(n, b + chunk);
-        try {
-            pool.emplace_back([&f, b, e]() { f(b, e); });
-        } catch (const std::exception&) {
-            f(b, e);
-        }
-    }
-    f(0, std::min(n, chunk));
     for (auto& th : pool) th.join();
 }
 
@@ -886,7 +863,7 @@ static uint32_t add_image(noor_payload_handle* h, const noor_image& im, int32_t 
 enum : uint32_t { kBadIndex = 1u, kBadVertex = 2u, kBadMaterial = 4u };
 static uint32_t check_arrays(const noor_scene_desc* d) {
     std::atomic<uint32_t> bad{0u};
-    parallel_ranges(d->num_triangles, [&](size_t b, size_t e) {
+    parallel_ranges(d->num_triangles, 65536, 1024, [&](size_t b, size_t e) {
         uint32_t v = 0, n = 0, u = 0, m = 0;
         for (size_t i = 3 * b; i < 3 * e; ++i) {
             v = std::max(v, d->vindices[i]);
@@ -897,7 +874,7 @@ static uint32_t check_arrays(const noor_scene_desc* d) {
         if (v >= d->num_vertices || n >= d->num_normals || u >= d->num_uvs) bad |= kBadIndex;
         if (m >= d->num_materials) bad |= kBadMaterial;
     });
-    parallel_ranges(d->num_vertices, [&](size_t b, size_t e) {
+    parallel_ranges(d->num_vertices, 65536, 1024, [&](size_t b, size_t e) {
         bool finite = true;  // exponent bits not all ones
         for (size_t i = 4 * b; i < 4 * e; ++i) finite &= (f2u(d->vertices[i]) & 0x7f800000u) != 0x7f800000u;
         if (!finite) bad |= kBadVertex;

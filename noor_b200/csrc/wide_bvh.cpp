@@ -5,8 +5,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <thread>
 
+#include "host_threads.h"
 #include "noor_b200.h"
 
 namespace nb {
@@ -264,20 +264,6 @@ bool build_wide_tree(const uint32_t* nodes8, size_t nn, uint32_t root, int max_s
     return true;
 }
 
-namespace {
-
-// f(first, last) over [0, n) on the host threads
-template <class F>
-void parallel_ranges(size_t n, F f) {
-    const size_t threads = std::min<size_t>(std::max(1u, std::thread::hardware_concurrency()), 16);
-    if (n < (1u << 14) || threads == 1) return f((size_t)0, n);
-    std::vector<std::thread> pool;
-    for (size_t k = 0; k < threads; ++k) pool.emplace_back(f, n * k / threads, n * (k + 1) / threads);
-    for (auto& t : pool) t.join();
-}
-
-}  // namespace
-
 bool pack_wide_tree(const uint32_t* nodes8, WideTree& tree, size_t num_tris, const std::vector<uint32_t>& ident,
                     WideTreeDev& out) {
     out = WideTreeDev{};
@@ -352,7 +338,7 @@ bool pack_wide_tree(const uint32_t* nodes8, WideTree& tree, size_t num_tris, con
     }
     out.root_word = tree_word(tree.root);
     out.nodes.swap(tree.nodes);
-    parallel_ranges(n, [&](size_t b, size_t e) {
+    nbh::parallel_ranges(n, 2048, 16, [&](size_t b, size_t e) {
         for (size_t i = b; i < e; ++i) {
             WideNodeHost& h = out.nodes[i];
             for (int s = 0; s < 4; ++s) {

@@ -996,21 +996,20 @@ NB_D uint32_t rays_per_warp(uint32_t n) {
     return take > 4u ? 32u : take;
 }
 
-// The walks of the adjoint: the four-wide tree where the
-// scene has one and the binary walk's stack fits its capacity (else the binary
-// tree, whose stack overflow is reported at that capacity)
+// The walks of the adjoint's replay: the four-wide tree where the scene has one
+// and the binary walk's stack fits its capacity, else the binary tree (whose stack
+// overflow is reported at that capacity, and whose nodes may be of any number)
 template <int ISECT, bool EXT>
 NB_D bool path_closest(const DevScene& S, const float3& o, const float3& d, float& tmax, HitRec& rec,
                        const SmemStack& st, uint32_t* status) {
-    const bool binary = S.mega4 == 0u;
-    return trace_closest4<ISECT, EXT>(S, HeldRay{o, d}, tmax, rec, st, binary ? S.stack_cap : S.stack_cap4, binary,
-                                      status);
+    if (S.mega4 == 0u) return trace_closest<ISECT, EXT>(S, o, d, tmax, rec, st, status);
+    return trace_closest4<ISECT, EXT>(S, HeldRay{o, d}, tmax, rec, st, S.stack_cap4, false, status);
 }
 template <int ISECT, bool EXT>
 NB_D bool path_any(const DevScene& S, const float3& o, const float3& d, float tmax, const SmemStack& st,
                    uint32_t* status) {
-    const bool binary = S.mega4 == 0u;
-    return trace_any4<ISECT, EXT>(S, HeldRay{o, d}, tmax, st, binary ? S.stack_cap : S.stack_cap4, binary, status);
+    if (S.mega4 == 0u) return trace_any<ISECT, EXT>(S, o, d, tmax, st, status);
+    return trace_any4<ISECT, EXT>(S, HeldRay{o, d}, tmax, st, S.stack_cap4, false, status);
 }
 
 }  // namespace nb

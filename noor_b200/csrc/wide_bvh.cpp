@@ -81,7 +81,7 @@ bool build_wide_tree(const uint32_t* nodes8, size_t nn, uint32_t root, int max_s
         out = WideTree{};
         return false;
     };
-    if (nn == 0 || nn >= (size_t)kWIndex || root >= nn) return fail("node count or root out of range");
+    if (nn == 0 || !ref_words_fit(nn) || root >= nn) return fail("node count or root out of range");
     const Tree T{nodes8, nn};
 
     // every node the traversal can reach, in post order (successors first),

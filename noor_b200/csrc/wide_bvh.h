@@ -52,6 +52,11 @@ constexpr uint32_t kWLeafShift = 26;
 constexpr uint32_t kWLeafMaxCount = 8;
 constexpr uint32_t kWLeafStart = (1u << kWLeafShift) - 1u;
 constexpr uint32_t kWInstance = kWRef | kWUntested;
+// Whether kWRef words can name the nodes of a tree: what build_wide_tree asks of
+// it, and what the walks of the binary tree by such words (trace_closest4 and
+// trace_any4, `binary`) do, whose words of larger indices would read as leaves
+// and instances
+constexpr bool ref_words_fit(size_t num_nodes) { return num_nodes < kWIndex; }
 // deepest stack a tree may need to be used (words per thread)
 constexpr int kWideMaxStack = 96;
 // meta[0] bits; the split axes of P, the left and the right child at bits

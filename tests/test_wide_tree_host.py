@@ -88,3 +88,32 @@ def _program(tmp_path, text, name):
 def test_packing_without_threads(tmp_path):
     out = _program(tmp_path, THREADS, "threads")
     assert out.returncode == 0 and out.stdout.split() == ["same"], (out.returncode, out.stdout, out.stderr)
+
+
+WORDS = r"""
+#include <cstdio>
+#include <string>
+#include "wide_bvh.h"
+int set_error(int code, const std::string&) { return code; }
+void clear_error() {}
+int main() {
+    using namespace nb;
+    // how the walks read a kWRef word: a leaf, an instance, else a node
+    auto node = [](uint32_t w) { return (w & (kWUntested | kWLeaf)) != kWLeaf && !(w & kWUntested) ? w & kWIndex : kWNone; };
+    for (size_t n : {(size_t)1, (size_t)2, (size_t)kWIndex - 1, (size_t)kWIndex, (size_t)kWIndex + 1, (size_t)kWLeaf + 6,
+                     (size_t)kWUntested + 1, (size_t)1 << 31, (size_t)0xFFFFFFFFu}) {
+        const uint32_t last = (uint32_t)(n - 1);
+        if (ref_words_fit(n) && node(kWRef | last) != last) return 2;
+        WideTree tree;
+        if (!ref_words_fit(n) && build_wide_tree(nullptr, n, 0, kWideMaxStack, tree, nullptr)) return 3;
+    }
+    if (!ref_words_fit((size_t)kWIndex - 1)) return 4;
+    puts("same");
+}
+"""
+
+
+def test_words_of_large_trees(tmp_path):
+    """node indices beyond a word's 29 bits are kept out of the walks that go by words"""
+    out = _program(tmp_path, WORDS, "words")
+    assert out.returncode == 0 and out.stdout.split() == ["same"], (out.returncode, out.stdout, out.stderr)

@@ -417,8 +417,8 @@ static int adjoint_run(const noor_adjoint_desc* desc, int mode, float* image, co
     const bool wt = S.isect == NOOR_ISECT_WATERTIGHT;
     const RadKernel kr = wt ? adj_radiance<NOOR_ISECT_WATERTIGHT> : adj_radiance<NOOR_ISECT_REF_WALD>;
     const GradKernel kg = wt ? adj_gradient<NOOR_ISECT_WATERTIGHT> : adj_gradient<NOOR_ISECT_REF_WALD>;
-    e = cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    e = allow_stacks(kr, kAdjBlock);
+    if (e == cudaSuccess) e = allow_stacks(kg, kAdjBlock);
     int per_sm = 1;
     if (e == cudaSuccess && mode == 1) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kg, kAdjBlock, sm);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint setup");

@@ -485,7 +485,7 @@ static int run_staged(Context& C, const DevScene& S, const AdjParams& P, int mod
     float4* Lbuf = record ? nullptr : (float4*)(p + lb);
     constexpr int trav = 64;
     const size_t sm = (size_t)S.stack_words * trav * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute(adj_trace<ISECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_stacks(adj_trace<ISECT>, trav);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint setup");
     for (uint32_t c0 = 0; c0 < P.spp; c0 += chunk) {
         W.frames = std::min(chunk, P.spp - c0);

@@ -1377,17 +1377,21 @@ int GpuPayload::trees(const std::vector<GpuMesh>& meshes, const GpuBvhParams& bp
         (e = dalloc(s, b_gcnt, max_large * 3 * P.nb, &d_gcnt)) || (e = dalloc(s, b_meshoff, M, &d_meshoff)))
         return fail("allocation", e);
 
-    // kernel shared memory
-    const SmallSmem tiny_l = small_layout(P.nb, kTinyCap, 32), small_l = small_layout(P.nb, kSmallCap, 256);
-    const size_t bin_smem = (size_t)3 * P.nb * kKeys * 8 + (size_t)3 * P.nb * 4 + (size_t)2 * 3 * P.nb * 4;
-    const size_t dec_smem = (size_t)4 * 3 * P.nb * sizeof(DBox) + (size_t)2 * 3 * P.nb * 4 + 3 * sizeof(AxisBest) +
-                            (size_t)2 * 3 * P.nb * 4;
-    if ((e = cudaFuncSetAttribute(k_split<32, kTinyCap>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tiny_l.total)) ||
-        (e = cudaFuncSetAttribute(k_split<256, kSmallCap>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)small_l.total)) ||
-        (e = cudaFuncSetAttribute(k_bin_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bin_smem)) ||
-        (e = cudaFuncSetAttribute(k_decide_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dec_smem)))
+    // kernel shared memory.  The limits belong to the kernels, not to the build:
+    // always what the most bins need, or a build of fewer would refuse the
+    // launches of another one on another thread
+    auto tiny_smem = [](uint32_t nb) { return small_layout(nb, kTinyCap, 32).total; };
+    auto small_smem = [](uint32_t nb) { return small_layout(nb, kSmallCap, 256).total; };
+    auto bin_smem = [](size_t nb) { return 3 * nb * kKeys * 8 + 3 * nb * 4 + 2 * 3 * nb * 4; };
+    auto dec_smem = [](size_t nb) {
+        return 4 * 3 * nb * sizeof(DBox) + 2 * 3 * nb * 4 + 3 * sizeof(AxisBest) + 2 * 3 * nb * 4;
+    };
+    auto allow = [](auto* kernel, size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    if ((e = allow(k_split<32, kTinyCap>, tiny_smem(kMaxBins))) ||
+        (e = allow(k_split<256, kSmallCap>, small_smem(kMaxBins))) || (e = allow(k_bin_large, bin_smem(kMaxBins))) ||
+        (e = allow(k_decide_large, dec_smem(kMaxBins))))
         return fail("shared memory", e);
 
     // inputs and the roots (records 0..M-1, one task per mesh)
@@ -1433,9 +1437,9 @@ int GpuPayload::trees(const std::vector<GpuMesh>& meshes, const GpuBvhParams& bp
             (e = cudaStreamSynchronize(s)))
             return fail("classify", e);
         if (h.n_tiny)
-            k_split<32, kTinyCap><<<h.n_tiny, 32, tiny_l.total, s>>>(d_tasks[cur], d_tiny, d_box, d_order, P, o);
+            k_split<32, kTinyCap><<<h.n_tiny, 32, tiny_smem(P.nb), s>>>(d_tasks[cur], d_tiny, d_box, d_order, P, o);
         if (h.n_small)
-            k_split<256, kSmallCap><<<h.n_small, 256, small_l.total, s>>>(d_tasks[cur], d_small, d_box, d_order, P,
+            k_split<256, kSmallCap><<<h.n_small, 256, small_smem(P.nb), s>>>(d_tasks[cur], d_small, d_box, d_order, P,
                                                                          o);
         if (h.n_large) {
             if (h.n_large > max_large) {
@@ -1469,8 +1473,8 @@ int GpuPayload::trees(const std::vector<GpuMesh>& meshes, const GpuBvhParams& bp
                 (e = cudaMemcpyAsync(d_c0, c0.data(), 4 * c0.size(), cudaMemcpyHostToDevice, s)))
                 return fail("chunk table", e);
             k_init_large_keys<<<(nbins + 255) / 256, 256, 0, s>>>(d_gkeys, d_gcnt, nbins);
-            k_bin_large<<<nc, 256, bin_smem, s>>>(d_tasks[cur], d_large, d_chunks, d_box, d_order, P, d_gkeys, d_gcnt);
-            k_decide_large<<<h.n_large, 32, dec_smem, s>>>(d_tasks[cur], d_large, P, d_gkeys, d_gcnt, d_splits, o);
+            k_bin_large<<<nc, 256, bin_smem(P.nb), s>>>(d_tasks[cur], d_large, d_chunks, d_box, d_order, P, d_gkeys, d_gcnt);
+            k_decide_large<<<h.n_large, 32, dec_smem(P.nb), s>>>(d_tasks[cur], d_large, P, d_gkeys, d_gcnt, d_splits, o);
             k_count_large<<<nc, 256, 0, s>>>(d_tasks[cur], d_large, d_chunks, d_splits, d_box, d_order, d_ctrue);
             k_scan_emit_large<<<(h.n_large + 63) / 64, 64, 0, s>>>(d_tasks[cur], d_large, h.n_large, d_c0, d_ctrue,
                                                                   d_cbefore, d_splits, P, o);

@@ -257,7 +257,8 @@ void apply_spec(SceneState& st, const noor_spec& s) {
     D.isect = s.intersector;
     D.film_mode = s.film_mode;
     int cap = (int)s.bvh_height + (int)st.max_mesh_leaf + 4;
-    D.stack_cap = cap < 16 ? 16 : (cap > 96 ? 96 : cap);
+    static_assert(kWideMaxStack == kMaxStackWords, "the deepest walk stack");
+    D.stack_cap = std::min(std::max(cap, 16), kMaxStackWords);
     // the four-wide tree serves the root it was built from
     const bool wide = st.wide_nodes && s.bvh_root_node == st.wide_root;
     D.nodes4 = wide ? st.wide_nodes : nullptr;

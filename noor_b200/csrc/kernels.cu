@@ -306,7 +306,7 @@ static cudaError_t launch_trace(const DevScene& S, bool wide, const noor_ray* ra
     const size_t sm = (size_t)S.stack_words * kTraceBlock * sizeof(uint32_t);
     const uint32_t grid = (uint32_t)((n + kTraceBlock - 1) / kTraceBlock);
     auto go = [&](auto kern) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_stacks(kern, kTraceBlock);
         if (e != cudaSuccess) return e;
         kern<<<grid, kTraceBlock, sm, s>>>(S, rays, out, n, status);
         return cudaGetLastError();

@@ -1,9 +1,21 @@
 // Host-visible launchers of the render and parity kernels.
 #pragma once
+#include <cuda_runtime.h>
+
 #include "scene_dev.cuh"
 
 namespace nb {
 
+// The most words a thread's walk stack has (DevScene::stack_words), and what every
+// launch of a kernel with such stacks allows of dynamic shared memory: the limit
+// belongs to the kernel, not to the launch or the context, so a smaller one set
+// for one scene would refuse a deeper scene's launch on another thread.
+constexpr int kMaxStackWords = 96;
+template <class K>
+cudaError_t allow_stacks(K* kernel, int threads) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kMaxStackWords * threads * (int)sizeof(uint32_t));
+}
 constexpr int kMegaBlock = 128;
 constexpr int kTraceBlock = 128;
 // resident blocks per SM of the small frames' kernel

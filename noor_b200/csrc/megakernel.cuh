@@ -113,7 +113,7 @@ cudaError_t launch_megakernel_isect(const DevScene& S, const DevCamera& C, const
     const size_t sm = (size_t)S.stack_cap * kMegaBlock * sizeof(uint32_t);
     const bool ext = ext_kernels(S, C);
     auto go = [&](auto kern) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_stacks(kern, kMegaBlock);
         if (e != cudaSuccess) return e;
         kern<<<grid, kMegaBlock, sm, s>>>(S, C, a);
         return cudaGetLastError();

@@ -12,7 +12,7 @@ template <int ISECT, bool EXT, bool DIFF>
 cudaError_t run_stages(const DevScene& S, const DevCamera& C, const StageDev& W, int sm_count, uint64_t* launches,
                        cudaStream_t s) {
     const size_t sm = (size_t)S.stack_words * kStageTrav * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute(st_trace<ISECT, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_stacks(st_trace<ISECT, EXT>, kStageTrav);
     if (e != cudaSuccess) return e;
     const uint32_t all = (W.paths + 255) / 256;
     // Two paths a warp until there are paths enough, where a walk is all that a

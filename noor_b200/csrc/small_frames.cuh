@@ -72,7 +72,7 @@ cudaError_t launch_small_isect(const DevScene& S, const DevCamera& C, const Mega
     const uint32_t grid = (warps + kMegaBlock / 32 - 1) / (kMegaBlock / 32);
     const size_t sm = (size_t)S.stack_words * kMegaBlock * sizeof(uint32_t);
     auto go = [&](auto kern) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_stacks(kern, kMegaBlock);
         if (e != cudaSuccess) return e;
         kern<<<grid, kMegaBlock, sm, s>>>(S, C, a, lanes);
         return cudaGetLastError();

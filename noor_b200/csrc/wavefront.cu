@@ -1098,7 +1098,7 @@ int wavefront_render(Context& C, const noor_wf_frame* frames, uint32_t n_frames,
         return set_error(NOOR_ERR_INVALID, "wavefront: shade_regs must be 0, 80 or 128");
     L.shade_wide_regs = P.shade_regs == 128;
     for (WfTravKernel k : {L.extend, L.shadow}) {
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+        e = allow_stacks(k, NB_TRAV_THREADS);
         if (e != cudaSuccess) return cuda_fail(e, "wavefront smem");
     }
     if (ms_out) cudaEventRecord(C.events[6], s);

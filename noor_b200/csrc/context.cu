@@ -415,6 +415,7 @@ int upload_scene(Context& C, const noor_payload* P, const noor_hosek_sky* H, con
     DevScene& D = st.dev;
     std::memset(&D, 0, sizeof(D));
     const size_t nt = P->num_triangles, nn = P->num_bvh_nodes, nv = P->num_vertices, ni = P->num_instances;
+    const std::vector<uint32_t> ident = identity_instances(P);
     // nodes: interleave the two uint4 arrays
     {
         std::vector<DevNode> h(nn);
@@ -432,7 +433,6 @@ int upload_scene(Context& C, const noor_payload* P, const noor_hosek_sky* H, con
         // where it qualifies); a tree it does not suit keeps the binary
         // traversal
         static_assert(sizeof(DevNode4) == sizeof(WideNodeHost), "device wide node");
-        const std::vector<uint32_t> ident = identity_instances(P);
         const uint32_t* words = reinterpret_cast<const uint32_t*>(h.data());
         WideTree wt;
         WideTreeDev wd;
@@ -491,7 +491,6 @@ int upload_scene(Context& C, const noor_payload* P, const noor_hosek_sky* H, con
                 std::memcpy(&x[i].nrm[r], P->normal_row[r] + 4 * i, 16);
             }
         if ((rc = st.upload((void**)&D.xforms, x.data(), ni * sizeof(DevXform), "transforms"))) return rc;
-        const std::vector<uint32_t> ident = identity_instances(P);
         if ((rc = st.upload((void**)&D.xf_ident, ident.data(), ident.size() * 4, "identity instances"))) return rc;
     }
     {

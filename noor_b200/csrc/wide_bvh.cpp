@@ -90,6 +90,7 @@ bool build_wide_tree(const uint32_t* nodes8, size_t nn, uint32_t root, int max_s
     std::vector<uint8_t> state(nn, 0);  // 0 new, 1 on the path, 2 done
     std::vector<uint8_t> pure(nn, 0);
     std::vector<uint32_t> post;
+    post.reserve(nn);
     {
         std::vector<std::pair<uint32_t, uint32_t>> path;  // node, next successor
         path.emplace_back(root, 0u);
@@ -119,6 +120,8 @@ bool build_wide_tree(const uint32_t* nodes8, size_t nn, uint32_t root, int max_s
     }
 
     out.map.assign(nn, kWNone);
+    out.nodes.reserve(nn / 4);
+    out.node.reserve(nn / 4);
     std::vector<uint32_t> work;
     bool deferred = false;
     auto get_wide = [&](uint32_t n) -> uint32_t {
@@ -186,20 +189,6 @@ bool build_wide_tree(const uint32_t* nodes8, size_t nn, uint32_t root, int max_s
             }
         }
         h.meta[0] = flags;
-        // the visiting order of the four slots for each ray octant (bit a of
-        // the octant: direction component a <= 0): the near side of P's split
-        // axis first, within it the near side of an expanded child's; two
-        // bits per slot, first visited lowest, one byte per octant
-        for (uint32_t o = 0; o < 8; ++o) {
-            const bool right_first = (o >> T.axis(P)) & 1u;
-            const uint32_t ax_l = (flags >> 6) & 3u, ax_r = (flags >> 8) & 3u;
-            const bool swap_l = (flags & kW4ExpandL) && ((o >> ax_l) & 1u);
-            const bool swap_r = (flags & kW4ExpandR) && ((o >> ax_r) & 1u);
-            const uint32_t l = swap_l ? 0x1u : 0x4u;  // slots (1,0) or (0,1)
-            const uint32_t r = swap_r ? 0xBu : 0xEu;  // slots (3,2) or (2,3)
-            const uint32_t order = right_first ? (r | l << 4) : (l | r << 4);
-            h.meta[1 + o / 4] |= order << (8 * (o % 4));
-        }
         out.nodes[out.map[P]] = h;
     }
 

@@ -66,8 +66,7 @@ constexpr uint32_t kW4ExpandL = 2u;  // slots 0, 1 hold the left child's childre
 constexpr uint32_t kW4ExpandR = 4u;  // slots 2, 3 hold the right child's children
 
 // 128 bytes: the four entry boxes as structure of arrays, the entry words,
-// and meta = {flags and axes, slot order for ray octants 0-3, for octants
-// 4-7, 0}
+// and meta = {flags and axes, 0, 0, 0}
 struct WideNodeHost {
     float lo[3][4];
     float hi[3][4];

@@ -354,7 +354,8 @@ int cuda_path_tracer(unsigned int* frame_count);
 /* path_tracer.cuh:148 / path_tracer.cu:102-130: write the sky texture (and,
  * with MIS on, red importance samples) into the film, then ++*frame_count. */
 int debug_skydome(unsigned int* frame_count, int width, int height);
-/* path_tracer.cuh:149: free the current context and all device memory. */
+/* path_tracer.cuh:149: free the current context and all device memory (but see
+ * noor_workspace_limit for what the device's pool keeps). */
 int device_free_memory(void);
 /* path_tracer.cuh:150: hit point of the centre pixel's primary ray from the
  * last frame (w = 1 if it hit, 0 otherwise). */
@@ -384,7 +385,10 @@ int noor_render_frames(unsigned int* frame_count, unsigned int n_frames);
  * of the limit backward, for at most 2^21 paths and 4 GiB at a time (1.6 GB for
  * 512 x 512 pixels, 16 samples and 4 bounces).  With less, or where the device
  * has no more, they take fewer frames or samples at a time, and where one does
- * not fit, the kernels that need no such memory. */
+ * not fit, the kernels that need no such memory.  The staged renderer's comes
+ * from the device's default pool, which keeps up to 4 GiB for the next context
+ * (and the next noor_build_payload_gpu) when a context goes; this call gives
+ * back what the pool holds unused. */
 int noor_workspace_limit(size_t bytes);
 /* Which kernels the current context renders its frames and its adjoint with,
  * to compare them with each other: by default (AUTO) the library chooses by

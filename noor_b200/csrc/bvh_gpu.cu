@@ -1144,7 +1144,9 @@ struct TimingEvents {
         if (b) cudaEventDestroy(b);
     }
 };
-static void keep_pool() {
+}  // namespace
+
+void keep_pool() {
     int dev = 0;
     cudaMemPool_t pool;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess) return;
@@ -1154,8 +1156,6 @@ static void keep_pool() {
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
 }
-
-}  // namespace
 
 // a host thread for copies from and to pageable memory, which hold up the
 // thread that issues them; where none can be had the caller does them itself

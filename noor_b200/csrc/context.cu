@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "bvh_gpu.h"
 #include "host_common.h"
 #include "kernels.h"
 #include "runtime.h"
@@ -785,6 +786,7 @@ extern "C" int load_cuda_data(const noor_payload* payload, const noor_hosek_sky*
     cudaDeviceGetAttribute(&C->sm_count, cudaDevAttrMultiProcessorCount, C->device);
     e = cudaStreamCreateWithFlags(&C->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "stream");
+    nbg::keep_pool();
     for (auto& ev : C->events)
         if ((e = cudaEventCreate(&ev)) != cudaSuccess) return cuda_fail(e, "event");
     if ((e = cudaMalloc((void**)&C->lookat, 16)) != cudaSuccess) return cuda_fail(e, "lookat");
@@ -883,7 +885,12 @@ extern "C" int noor_workspace_limit(size_t bytes) {
         C->adj_buf = nullptr;
         C->adj_bytes = 0;
     }
-    return sync_and_check(*C, "noor_workspace_limit");
+    if ((rc = sync_and_check(*C, "noor_workspace_limit"))) return rc;
+    // and what earlier contexts left with the device's pool
+    cudaMemPool_t pool;
+    cudaError_t e = cudaDeviceGetDefaultMemPool(&pool, C->device);
+    if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
+    return e == cudaSuccess ? NOOR_OK : cuda_fail(e, "noor_workspace_limit");
 }
 
 extern "C" int noor_route(int frames, int adjoint) {

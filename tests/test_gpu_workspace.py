@@ -126,3 +126,35 @@ def test_a_full_device():
         hold.clear()
         torch.cuda.empty_cache()
         r.close()
+
+
+POOL = r"""
+import ctypes as C, sys
+import torch
+from noor_b200 import _capi, scenes
+torch.zeros(1, device="cuda")
+free = lambda: (torch.cuda.synchronize(), torch.cuda.mem_get_info()[0] >> 20)[1]
+make = lambda: scenes.Renderer(scenes.room_scene(width=1024, height=1024))
+r = make(); r.close()
+at = [free()]
+r = make(); r.render(1); r.close()
+at.append(free())                      # the next context's: some 240 MB
+r = make(); r.render(1)
+_capi.call("noor_workspace_limit", C.c_size_t(0))
+r.close()
+at.append(free())
+print(*at)
+"""
+
+
+def test_the_pool_keeps_and_gives_back():
+    """host-built payloads only: what a context gives back serves the next one, until it is asked for"""
+    import subprocess
+    import sys
+    from pathlib import Path
+    out = subprocess.run([sys.executable, "-c", POOL], capture_output=True, text=True, timeout=300,
+                         cwd=Path(__file__).resolve().parents[1])
+    assert out.returncode == 0, out.stderr[-2000:]
+    before, kept, after = map(int, out.stdout.split())
+    assert before - kept >= 200
+    assert before - after <= 64

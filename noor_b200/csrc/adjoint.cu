@@ -19,6 +19,7 @@
 #include <cstring>
 
 #include "host_common.h"
+#define NB_ADJOINT_ROUNDING  // as adjoint_stages.cu
 #include "adjoint.cuh"
 
 namespace nb {
@@ -163,7 +164,7 @@ NB_D float3 replay(const PathCtx& C, uint32_t pix, uint32_t frame, const DevCame
         HitRec rec;
         if (!path_closest<ISECT, false>(S, o, d, tmax, rec, C.st, C.status)) {
             if (S.sky_on && (bounce == 0 || spec)) {
-                const float3 dir = normalize_fast(d);
+                const float3 dir = d * rsqrtf(stage_length2(d));
                 float3 Le;
                 Bilerp bl;
                 const bool env = S.sky_type == NOOR_SKY_HDR;
@@ -188,7 +189,7 @@ NB_D float3 replay(const PathCtx& C, uint32_t pix, uint32_t frame, const DevCame
             break;
         }
         Isect I;
-        make_isect<ISECT, false>(S, o, d, tmax, rec, I);
+        make_isect<ISECT, false, true>(S, o, d, tmax, rec, I);
         if (I.mtype & kEmitterMat) {
             if (bounce == 0 || spec) {
                 if (I.mtype & NOOR_MESHLIGHT) {

@@ -463,8 +463,9 @@ NB_D RayDiff spawn_diff(const Isect& I, const HitDiff& h, const RayDiff& in, con
 // Builds the hit record of CudaIntersection (intersection.cuh:319-377).
 // With `to`, also the texture coordinates and derivatives of TangentOut
 // (I.uv: the barycentrics on an emitter, whose record stops before them).
-// STAGE: for the staged renderer, whose shading has to round as the
-// megakernel's: there the length of d is z z + (y y + x x), each sum fused.
+// STAGE: for the kernels that cuda_path_tracer renders with, which have to round
+// alike wherever the direction comes from: the length of d is z z + (y y + x x),
+// each sum fused, as the compiler chose in the megakernel.
 NB_D float stage_length2(const float3& d) {
     return __fmaf_rn(d.z, d.z, __fmaf_rn(d.y, d.y, __fmul_rn(d.x, d.x)));
 }
@@ -534,13 +535,14 @@ NB_D float3 path_radiance(const DevScene& S, float3 o, float3 d, Rng& rng, const
         HitRec rec;
         rs.ext++;
         if (!trace_primary<ISECT, EXT, WIDE>(S, HeldRay{o, d}, tmax, rec, st, status)) {
-            if (S.sky_on && (bounce == 0 || spec_bounce)) L += beta * env_eval<EXT>(S, normalize_fast(d));
+            if (S.sky_on && (bounce == 0 || spec_bounce))
+                L += beta * env_eval<EXT>(S, d * rsqrtf(stage_length2(d)));
             break;
         }
         Isect I;
         TangentOut to;
         const bool tex = EXT && S.has_tex;
-        make_isect<ISECT, EXT>(S, o, d, tmax, rec, I, tex ? &to : nullptr);
+        make_isect<ISECT, EXT, true>(S, o, d, tmax, rec, I, tex ? &to : nullptr);
         if (bounce == 0 && first_hit) {
             *first_hit = I.p;
             *first_hit_valid = true;

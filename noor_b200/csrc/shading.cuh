@@ -235,10 +235,10 @@ NB_D float3 to_local(const Frame& F, const float3& v) { return f3(dot(v, F.s), d
 // The outgoing and the incoming direction of a BSDF in the shading frame.  The
 // compiler fuses the first two products of a dot product either way round,
 // depending on the code around it, and a path takes another turn where the
-// last bit moves; NB_ADJOINT_ROUNDING pins the choices it makes in the
-// adjoint's replay, for the file that evaluates the same paths in stages
-// (found by comparing the replay's sampled directions and pdfs with each of
-// the roundings; all of 20,000 glass samples agree with this one).
+// last bit moves; NB_ADJOINT_ROUNDING pins the choices it made in the adjoint's
+// replay, for the two files that evaluate the same paths, with a thread each and
+// in stages (found by comparing the replay's sampled directions and pdfs with
+// each of the roundings; all of 20,000 glass samples agree with this one).
 #ifdef NB_ADJOINT_ROUNDING
 NB_D float dot_xy(const float3& a, const float3& b) {   // (x x' + [y y']) + z z'
     return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));

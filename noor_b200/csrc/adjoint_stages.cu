@@ -414,7 +414,7 @@ static int run_staged(Context& C, const DevScene& S, const AdjParams& P, int mod
     *done = false;
     const uint32_t npix = C.cam.w * C.cam.h;
     if (S.bounces == 0 || S.bounces > 1024) return NOOR_OK;
-    if (!S.mega4 && !ref_words_fit(S.num_nodes)) return NOOR_OK;
+    if (!S.frames4 && !ref_words_fit(S.num_nodes)) return NOOR_OK;
     const bool record = mode == 1;
     const uint32_t verts = record ? S.bounces : 1u;
     // bytes a path takes below

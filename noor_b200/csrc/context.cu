@@ -270,7 +270,7 @@ void apply_spec(SceneState& st, const noor_spec& s) {
     D.reach4 = wide ? st.wide_reach : 0.0f;
     D.stack_cap4 = wide ? st.wide_cap : 0;
     D.closest4 = wide && st.wide_closest ? 1u : 0u;
-    D.mega4 = D.closest4 && st.wide_binary_need <= D.stack_cap ? 1u : 0u;
+    D.frames4 = D.closest4 && st.wide_binary_need <= D.stack_cap ? 1u : 0u;
     D.stack_words = std::max(D.stack_cap, D.stack_cap4);
 }
 

@@ -273,7 +273,7 @@ bool small_frames_fit(const DevScene& S, const DevCamera& C, const MegaArgs& a, 
 
 cudaError_t launch_small_frames(const DevScene& S, const DevCamera& C, const MegaArgs& a, int sm_count, cudaStream_t s) {
     // trees without a four-wide form: the megakernel's walks
-    if (!S.mega4) return launch_megakernel(S, C, a, s);
+    if (!S.frames4) return launch_megakernel(S, C, a, s);
     // Paths a warp, a power of two: 32, or fewer where that leaves warps to
     // spare.  Walks fill the resident warps (one frame under the sky of 97x61,
     // 32 / 8 / 4 paths a warp: 147 / 115 / 102 us); the larger code of the

@@ -168,7 +168,7 @@ int render_staged(Context& C, const DevScene& S, const MegaArgs& a, bool* done) 
     *done = false;
     const uint64_t npix = (uint64_t)C.cam.w * C.cam.h;
     if (npix > kStageMaxPaths || S.bounces == 0 || S.bounces > 1024) return NOOR_OK;
-    if (!S.mega4 && !ref_words_fit(S.num_nodes)) return NOOR_OK;
+    if (!S.frames4 && !ref_words_fit(S.num_nodes)) return NOOR_OK;
     StageDev W{};
     const uint32_t nb = stage_buffers(C, (uint32_t)npix, (uint32_t)std::min<uint64_t>(a.nframes, kStageMaxPaths / npix),
                                       S.bounces, S.has_bump != 0u, W);

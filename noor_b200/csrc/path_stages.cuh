@@ -200,7 +200,7 @@ NB_D void stage_extend(const DevScene& S, const DevCamera& C, const StageDev& W,
         float tmax = kInf;
         HitRec rec{0.0f, 0.0f, 0u, 0u, 0u};
         const StoredRay ray{W.o + i, W.d + i};
-        const bool binary = S.mega4 == 0u;
+        const bool binary = S.frames4 == 0u;
         if (!trace_closest4<ISECT, EXT>(S, ray, tmax, rec, stk, binary ? S.stack_cap : S.stack_cap4, binary, W.status)) {
             const bool sky = S.sky_on && (bounce == 0 || W.d[i].w != 0.0f);
             W.hit2[i] = make_uint2(0u, sky ? kStSky : kStDone);
@@ -348,7 +348,7 @@ NB_D void stage_occlude(const DevScene& S, const StageDev& W, uint32_t bounce, c
         const uint32_t q = base + lane;
         if (lane >= take || q >= n) continue;
         const StoredRay ray{W.sh_o + q, W.sh_d + q};
-        const bool binary = S.mega4 == 0u;
+        const bool binary = S.frames4 == 0u;
         if (trace_any4<ISECT, EXT>(S, ray, W.sh_o[q].w, stk, binary ? S.stack_cap : S.stack_cap4, binary, W.status))
             W.pend[2u * (size_t)W.keep * bounce + W.qshadow[q]].w = 0.0f;
     }

@@ -222,7 +222,7 @@ struct DevScene {
     float reach4;               // the largest coordinate of the tree's boxes
     int stack_cap4;
     uint32_t closest4;      // closest hit may use the four-wide tree
-    uint32_t mega4;         // so may the staged renderer and the adjoint: the binary walk's stack fits stack_cap too
+    uint32_t frames4;       // so may the small frames, the stages and the adjoint: the binary walk's stack fits stack_cap too
     int stack_words;
     // NOOR_ENV_REFERENCE: the reference's distribution tables (row r at
     // r * (rw + 1), the marginal at rh * (rw + 1)) and the environment as a

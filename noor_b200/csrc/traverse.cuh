@@ -845,7 +845,7 @@ NB_D bool trace_any4(const DevScene& S, const World& world, float tmax, const Sm
 // trace_closest.  Leaves are taken in the binary traversal's order.  A ref is
 // slab-tested when it is taken and a leaf when a triangle of it is hit, both
 // against the hit distance of the moment they were taken, as the binary
-// traversal tests them; the quantized boxes only skip what the binary
+// traversal tests them; the widened boxes only skip what the binary
 // traversal would find missed (its hit distance only shrinks, and a box
 // inside a missed box is missed).
 template <int ISECT, bool EXT, class World>
@@ -1002,13 +1002,13 @@ NB_D uint32_t rays_per_warp(uint32_t n) {
 template <int ISECT, bool EXT>
 NB_D bool path_closest(const DevScene& S, const float3& o, const float3& d, float& tmax, HitRec& rec,
                        const SmemStack& st, uint32_t* status) {
-    if (S.mega4 == 0u) return trace_closest<ISECT, EXT>(S, o, d, tmax, rec, st, status);
+    if (S.frames4 == 0u) return trace_closest<ISECT, EXT>(S, o, d, tmax, rec, st, status);
     return trace_closest4<ISECT, EXT>(S, HeldRay{o, d}, tmax, rec, st, S.stack_cap4, false, status);
 }
 template <int ISECT, bool EXT>
 NB_D bool path_any(const DevScene& S, const float3& o, const float3& d, float tmax, const SmemStack& st,
                    uint32_t* status) {
-    if (S.mega4 == 0u) return trace_any<ISECT, EXT>(S, o, d, tmax, st, status);
+    if (S.frames4 == 0u) return trace_any<ISECT, EXT>(S, o, d, tmax, st, status);
     return trace_any4<ISECT, EXT>(S, HeldRay{o, d}, tmax, st, S.stack_cap4, false, status);
 }
 

@@ -9,10 +9,10 @@
 // orders them by the ray's sign on P's and C's split axes visits leaves in
 // exactly the order of the binary traversal (noor/cuda/bvh.cuh:193-234).
 // Skipping C's own slab test changes no outcome: for a ray whose direction
-// components are all normal floats and whose origin is finite, the slab
-// test's per-axis intervals are monotone in the box bounds, so a box inside
-// C can only pass where C passes; other rays walk the binary tree below
-// that point, node by node.
+// components lie within 1e-18 .. 1e18 and whose origin within 1e12
+// (wide_degenerate in traverse.cuh), the slab test's per-axis intervals are
+// monotone in the box bounds, so a box inside C can only pass where C passes;
+// other rays walk the binary tree below that point, node by node.
 //
 // Entries whose slab test the binary traversal runs against a ray that may
 // differ from the one at P's visit (an entry without instance bits under a

@@ -172,6 +172,11 @@ def build_scene(args):
     return s, built, time.time() - t
 
 
+def tri_bytes(isect):
+    """bytes of a triangle test: Wald's first sector, or three vertices"""
+    return 32.0 if isect == 1 else 48.0
+
+
 def algorithmic_bytes(orc, cam, spp, isect, sample_pixels=20000, seed=0):
     """Bytes the path reads by the traversal/shading model: per traversal step
     32 B per node, per tested triangle 48 B (watertight: three vertices) or
@@ -192,7 +197,7 @@ def algorithmic_bytes(orc, cam, spp, isect, sample_pixels=20000, seed=0):
         tot += c
         paths += 2 * (p1 - int(b))
     ext, shadow, nodes, tris, inrange, sh_nodes, sh_tris, sh_inrange = [float(x) / paths for x in tot]
-    tri_b = 32.0 if isect == 1 else 48.0
+    tri_b = tri_bytes(isect)
 
     def trav(nd, tr, ir):
         return 32.0 * nd + tri_b * tr + (16.0 * ir if isect == 1 else 0.0)
@@ -781,12 +786,18 @@ def main():
             orc.close()
             if top_kernel == "wf_extend":
                 # traversal bytes of the extension rays + the slot state of every ray
+                tree = path.describe()["wavefront"]["tree"]
+                if tree in ("auto", "four-wide"):
+                    # the oracle walks the binary tree, so it has no count of the
+                    # four-wide tree's visits: triangles only
+                    counts["ext_traversal_bytes_per_path"] = counts["ext_tris_per_path"] * tri_bytes(r.spec.intersector)
+                    roof["algorithmic_bytes"] = "triangles tested and slot state; the four-wide tree's nodes are not in it"
                 alg = counts["ext_traversal_bytes_per_path"] * npaths + EXTEND_SLOT_BYTES * ext / args.steps
                 # the ncu capture is of the sky-lit scene
                 tr = profiled_traffic_per_ray() if args.workload == "sky" else None
                 traffic = tr * ext / args.steps / top_launches if tr else None
             elif top_kernel == "wf_shadow":
-                # traversal bytes of the shadow rays + the queue state of every one
+                # traversal bytes of the shadow rays (as if on the binary tree) + the queue state of every one
                 alg = counts["shadow_traversal_bytes_per_path"] * npaths + SHADOW_QUEUE_BYTES * shadow / args.steps
                 traffic = None
             else:

@@ -392,8 +392,10 @@ int noor_render_frames(unsigned int* frame_count, unsigned int n_frames);
 int noor_workspace_limit(size_t bytes);
 /* Which kernels the current context renders its frames and its adjoint with,
  * to compare them with each other: by default (AUTO) the library chooses by
- * the size of the work.  The results are the same.  A route that cannot serve
- * a call (no memory for the stages) leaves it to the library's choice.
+ * the size of the work.  The results are the same to the bit, but for the
+ * order of the gradients' sums.  A route that cannot serve a call (no memory for
+ * the stages, several samples of a pixel in one running mean with SMALL) leaves
+ * it to another.
  * frames: AUTO, MEGAKERNEL, STAGED or SMALL (a thread per path, on the
  * four-wide tree); adjoint: AUTO, REPLAY (a thread per
  * path) or STAGED. */

@@ -260,12 +260,12 @@ cudaError_t launch_megakernel(const DevScene& S, const DevCamera& C, const MegaA
 //   3     the room with a limit of 32, 384x288: 419 / 562 / 346 (512x512: 796 / 753 / 829)
 //   1     with the code of all lights, textures and bump maps, 5 bounces in the
 //         textured room: 192x144 329 / 291 / 271, 320x240 514 / 371 / 403
-//   4     the same with a limit of 32: 384x288 788 / 1179 / 648, 641x359 984 / 1310 / 948
+//   4.5   the same with limits of 16 and more, of 32: 384x288 788 / 1179 / 648, 641x359 984 / 1310 / 948
 bool small_frames_fit(const DevScene& S, const DevCamera& C, const MegaArgs& a, int sm_count) {
     const bool ext = ext_kernels(S, C), shallow = S.num_tris < 16384u;
     const uint64_t wave = (uint64_t)sm_count * kSmallBlocks(ext) * kMegaBlock;
     const uint32_t b = S.bounces;
-    const uint64_t half_waves = ext       ? (b < 8u ? 2 : b < 12u ? 3 : b < 24u ? 4 : 8)
+    const uint64_t half_waves = ext       ? (b < 8u ? 2 : b < 12u ? 3 : b < 16u ? 4 : 9)
                                 : shallow ? (b < 12u ? 3 : b < 24u ? 4 : 6)
                                           : (b < 4u ? 3 : b < 6u ? 4 : b < 12u ? 8 : b < 16u ? 12 : b < 32u ? 16 : 24);
     return 2 * (uint64_t)C.w * C.h * a.nframes <= wave * half_waves;
